@@ -160,6 +160,10 @@ struct GEntF {
   int32_t light_id;  // lights: registration index (Entity::light_id), which the reference
                      // uses as an index into the sorted list (directLight_radiance.h:541)
   // disk: u_length = radius, v_length = inner radius, n = the plane normal
+  // sphere: the FP32 bounds' anchor u, q = anchor - centre (high parts v, low
+  // parts n), c0 = |q|^2 - r^2 (high u_length, low v_length) and node_base =
+  // hemisphere (trace_fast.cuh)
+  // mesh: its bounds from u (lower) to v (upper)
 };
 
 // One entry of the light list in LightList::random_light_setup's order

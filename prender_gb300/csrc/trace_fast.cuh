@@ -67,9 +67,29 @@ __device__ __forceinline__ WRay make_wray(float3 o, float3 d) {
   return r;
 }
 
-// byte k of w as an exact float (0x4B0000qq is 2^23 + qq)
-__device__ __forceinline__ float qbyte(uint32_t w, int k) {
-  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + (uint32_t)k)) - 8388608.0f;
+// two FP32 values in one register pair: Blackwell's packed fma / add
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float o[2]) { asm("mov.b64 {%0, %1}, %2;" : "=f"(o[0]), "=f"(o[1]) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// bytes k and k + 1 of w as exact floats (0x4B0000qq is 2^23 + qq)
+__device__ __forceinline__ f32x2 qbytes2(uint32_t w, int k) {
+  return add2(pack2(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + (uint32_t)k)),
+                    __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7441u + (uint32_t)k))),
+              pack2(-8388608.0f, -8388608.0f));
 }
 
 // three-input minimum / maximum (one instruction on sm_100 and later)
@@ -121,33 +141,38 @@ __device__ __forceinline__ void wnode_visit(const WNode* __restrict__ n, const W
   const float bx = (a.x - r.o.x) * r.inv.x;
   const float by = (a.y - r.o.y) * r.inv.y;
   const float bz = (a.z - r.o.z) * r.inv.z;
+  const f32x2 sx2 = pack2(sx, sx), sy2 = pack2(sy, sy), sz2 = pack2(sz, sz);
+  const f32x2 bx2 = pack2(bx, bx), by2 = pack2(by, by), bz2 = pack2(bz, bz);
   // near and far planes per axis: the low planes are near for a positive direction
   const bool nx = r.oct & 1, ny = r.oct & 2, nz = r.oct & 4;
   const uint32_t nx0 = nx ? d.z : c.x, nx1 = nx ? d.w : c.y, fx0 = nx ? c.x : d.z, fx1 = nx ? c.y : d.w;
   const uint32_t ny0 = ny ? e.x : c.z, ny1 = ny ? e.y : c.w, fy0 = ny ? c.z : e.x, fy1 = ny ? c.w : e.y;
   const uint32_t nz0 = nz ? e.z : d.x, nz1 = nz ? e.w : d.y, fz0 = nz ? d.x : e.z, fz1 = nz ? d.y : e.w;
+  // two children per packed FP32 instruction: the kernel is bound by
+  // instruction issue, and fma / add on f32x2 round as the scalar ones do
   uint32_t hits = 0;
 #pragma unroll
-  for (int s = 0; s < 8; s++) {
+  for (int s = 0; s < 8; s += 2) {
     const int k = s & 3;
-    const float tnx = fmaf(qbyte(s < 4 ? nx0 : nx1, k), sx, bx);
-    const float tfx = fmaf(qbyte(s < 4 ? fx0 : fx1, k), sx, bx);
-    const float tny = fmaf(qbyte(s < 4 ? ny0 : ny1, k), sy, by);
-    const float tfy = fmaf(qbyte(s < 4 ? fy0 : fy1, k), sy, by);
-    const float tnz = fmaf(qbyte(s < 4 ? nz0 : nz1, k), sz, bz);
-    const float tfz = fmaf(qbyte(s < 4 ? fz0 : fz1, k), sz, bz);
-    const float tn = fmax3(tnx, tny, fmaxf(tnz, 0.0f));
-    const float tf = fmin3(tfx, tfy, fminf(tfz, tmax));
-    hits |= (tn <= tf) ? (1u << s) : 0u;
+    float tnx[2], tfx[2], tny[2], tfy[2], tnz[2], tfz[2];
+    unpack2(fma2(qbytes2(s < 4 ? nx0 : nx1, k), sx2, bx2), tnx);
+    unpack2(fma2(qbytes2(s < 4 ? fx0 : fx1, k), sx2, bx2), tfx);
+    unpack2(fma2(qbytes2(s < 4 ? ny0 : ny1, k), sy2, by2), tny);
+    unpack2(fma2(qbytes2(s < 4 ? fy0 : fy1, k), sy2, by2), tfy);
+    unpack2(fma2(qbytes2(s < 4 ? nz0 : nz1, k), sz2, bz2), tnz);
+    unpack2(fma2(qbytes2(s < 4 ? fz0 : fz1, k), sz2, bz2), tfz);
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const float tn = fmax3(tnx[j], tny[j], fmaxf(tnz[j], 0.0f));
+      const float tf = fmin3(tfx[j], tfy[j], fminf(tfz[j], tmax));
+      hits |= (tn <= tf) ? (1u << (s + j)) : 0u;
+    }
   }
   const uint32_t imask = em >> 24;
   uint32_t tm = 0;
-  if (hits & ~imask) {
-#pragma unroll
-    for (int s = 0; s < 8; s++) {
-      const uint32_t m = ((s < 4 ? (uint32_t)b.z : (uint32_t)b.w) >> (8 * (s & 3))) & 0xFFu;
-      tm |= ((hits >> s) & 1u) ? ((m >> 5) << (m & 31u)) : 0u;
-    }
+  for (uint32_t leaves = hits & ~imask; leaves; leaves &= leaves - 1u) {
+    const uint32_t m = __byte_perm((uint32_t)b.z, (uint32_t)b.w, __ffs(leaves) - 1u) & 0xFFu;
+    tm |= (m >> 5) << (m & 31u);
   }
   g.base = b.x;
   g.bits = permute_xor8(hits & imask, r.oct) | imask << 8;
@@ -277,6 +302,302 @@ __device__ __forceinline__ bool fast_circle(const GEntF& e, float3 o, float3 d, 
   return true;
 }
 
+// ---- spheres without FP64 ---------------------------------------------
+// GB300 issues one FP64 warp instruction per 16 clocks and SM (64 per
+// scheduler) whatever number of lanes is active, so the nine FP64 sphere
+// tests of a ray in the sphere Cornell box, not memory, bound such scenes
+// (FP64 pipe 85 % busy).  The FP64 test is kept for the spheres that can
+// still be the answer; the others are ruled out in FP32 with error bounds:
+// along the ray the test solves F(t) = t^2 + 2 b t + c = 0, with b = d.(o-C)
+// and c = |o-C|^2 - r^2.  From an anchor A (the centre, or for a sphere much
+// larger than the scene the point of its surface nearest to the scene, which
+// keeps the cancellation out of c) with w = o - A and q = A - C:
+//   b = d.w + d.q,  c = w.w + 2 w.q + c0,  c0 = |q|^2 - r^2.
+// A is a float triple exactly; q and c0 carry FP32 high and low parts
+// (GEntF::v / n, u_length / v_length).  kSphErr = 16 rounding units bounds
+// each sum's error relative to its terms' magnitudes.
+constexpr float kSphErr = 1.0e-6f;
+constexpr float kSphNear = 1.0e-5f;  // above the test's own threshold of 1e-6
+
+struct SphF {
+  float b, c, eb, ec;  // coefficients and their error bounds
+};
+
+__device__ __forceinline__ SphF sph_coeffs(const GEntF& e, float3 o, float3 d, float dmax) {
+  const float3 w = o - f3(e.u[0], e.u[1], e.u[2]), q = f3(e.v[0], e.v[1], e.v[2]);
+  const float m = fabsf(w.x) + fabsf(w.y) + fabsf(w.z), Q = fabsf(q.x) + fabsf(q.y) + fabsf(q.z);
+  SphF f;
+  f.b = dot(d, w) + dot(d, q);
+  f.c = dot(w, w) + 2.0f * dot(w, q) + e.u_length;
+  f.eb = kSphErr * (m + Q) * dmax;
+  f.ec = kSphErr * (m * m + 2.0f * m * Q + fabsf(e.u_length));
+  return f;
+}
+__device__ __forceinline__ float sph_val(const SphF& f, float t) { return fmaf(t, t + 2.0f * f.b, f.c); }
+__device__ __forceinline__ float sph_err(const SphF& f, float t) {
+  return f.ec + 2.0f * t * f.eb + kSphErr * (t * (t + 2.0f * fabsf(f.b)) + fabsf(f.c));
+}
+
+// c to about 1e-13 of its terms (two-float sums and products: Dekker 1971,
+// Knuth; the products' errors by fma), for an origin on the sphere itself
+// (where a ray that just left it starts), whose c FP32 cannot tell from 0
+__device__ __forceinline__ void two_add(float& s, float& e, float x) {
+  const float t = __fadd_rn(s, x), z = __fsub_rn(t, s);
+  e += __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(x, z));
+  s = t;
+}
+__device__ __forceinline__ float sph_c_refined(const GEntF& e, float3 o) {
+  float s = e.u_length, err = e.v_length;
+  const float oo[3] = {o.x, o.y, o.z};
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const float A = e.u[a];
+    float w = oo[a], wl = 0.0f;  // w + wl = o - A exactly
+    two_add(w, wl, -A);
+    float y = w, yl = wl + 2.0f * e.n[a];  // y + yl = w + 2 q
+    two_add(y, yl, 2.0f * e.v[a]);
+    const float p = __fmul_rn(w, y);
+    two_add(s, err, p);
+    err += fmaf(w, y, -p) + (w * yl + wl * y);
+  }
+  return s + err;
+}
+
+// rules sphere e out: no hit of it can lie below the limit T
+__device__ __forceinline__ bool sph_reject(const SphF& f, float T) {
+  const float v = sph_val(f, T), ev = sph_err(f, T);
+  if (f.c < -f.ec) return v < -ev;  // the origin is inside: the exit lies beyond T
+  if (f.c > f.ec) {
+    if (f.b > f.eb) return true;  // outside and behind
+    const float D = f.b * f.b - f.c;
+    if (D < -(2.0f * fabsf(f.b) * f.eb + f.eb * f.eb + f.ec + kSphErr * f.b * f.b)) return true;  // passes by
+    return v > ev && T < -f.b - f.eb;  // the entry lies beyond T
+  }
+  return false;
+}
+
+// the same for an origin on the sphere: the near root lies below the test's
+// threshold (so the far one would be returned) and the far one beyond T
+__device__ __forceinline__ bool sph_reject_surface(const GEntF& e, const SphF& f, float3 o, float T) {
+  const float c = sph_c_refined(e, o);
+  // error of c (1e-12 of its terms), and half of F(1e-6) - c = 2 b 1e-6 as room
+  const float room = 1.0e-6f * fabsf(f.b) - 1.0e-6f * f.ec;
+  if (!(room > 0.0f)) return false;
+  if (f.b > f.eb) return c > -room;  // leaving outward: both roots below 1e-6
+  if (f.b < -f.eb) return c < room && sph_val(f, T) < -sph_err(f, T);
+  return false;
+}
+
+// an upper bound of sphere e's hit distance, where it is certain to be hit
+// (the caller excludes hemispheres); 3e38 where it is not
+__device__ __forceinline__ float sph_upper(const SphF& f) {
+  const float D = f.b * f.b - f.c;
+  if (!(D > 0.0f)) return 3.0e38f;
+  const float s = sqrtf(D);
+  const float vn = sph_val(f, kSphNear), en = sph_err(f, kSphNear);
+  if (f.c < -f.ec) {
+    const float t = (f.b <= 0.0f ? s - f.b : __fdividef(-f.c, f.b + s)) * 1.001f + 1.0e-3f;
+    return (vn < -en && sph_val(f, t) > sph_err(f, t)) ? t : 3.0e38f;
+  }
+  if (f.c > f.ec && f.b < -f.eb) {
+    const float t = __fdividef(f.c, s - f.b) * 1.001f + 1.0e-3f;
+    return (vn > en && sph_val(f, t) < -sph_err(f, t)) ? t : 3.0e38f;
+  }
+  return 3.0e38f;
+}
+
+// The run of consecutive spheres of the entity list from i on (i moves past
+// it): the closest one below h.t, as the FP64 test of each in list order
+// finds it.  Spheres ruled out by the FP32 bounds lie beyond a certain hit
+// of another one (by more than a float rounding), so leaving them out does
+// not change which sphere wins nor its distance.
+__device__ __forceinline__ void sphere_run_closest(const DevScene& S, int& i, float3 o, float3 d, FastHit& h) {
+  const int first = i;
+  const float dmax = fmaxf(1.0f, fmaxf(fabsf(d.x), fmaxf(fabsf(d.y), fabsf(d.z))));
+  unsigned long long left = 0;  // spheres not ruled out (bit: index in the run)
+  float T = h.t;
+  for (; i < S.n_ents && S.entf[i].type == PR_ENT_SPHERE; i++) {
+    const GEntF& e = S.entf[i];
+    const SphF f = sph_coeffs(e, o, d, dmax);
+    if (sph_reject(f, T)) continue;
+    left |= 1ull << (i - first);
+    if (!e.node_base) T = fminf(T, sph_upper(f));  // node_base: a hemisphere
+  }
+  while (left) {
+    const int k = first + __ffsll((long long)left) - 1;
+    left &= left - 1;
+    const GEntF& e = S.entf[k];
+    const SphF f = sph_coeffs(e, o, d, dmax);
+    const float Tk = fminf(T, h.t);
+    if (sph_reject(f, Tk) || (fabsf(f.c) <= f.ec && sph_reject_surface(e, f, o, Tk))) continue;
+    float t, rest;
+    if (fast_sphere(S.ents[k], o, d, h.t, t, rest) && t < h.t) {
+      h.t = t;
+      h.ent = k;
+      h.slot = -1;
+      h.u = rest;
+      h.v = 0.0f;
+    }
+  }
+}
+
+// the run's any-hit query: a sphere hit below tmax, or -1
+__device__ __forceinline__ int sphere_run_any(const DevScene& S, int& i, float3 o, float3 d, float tmax) {
+  const float dmax = fmaxf(1.0f, fmaxf(fabsf(d.x), fmaxf(fabsf(d.y), fabsf(d.z))));
+  const int first = i;
+  unsigned long long left = 0;
+  int found = -1;
+  for (; i < S.n_ents && S.entf[i].type == PR_ENT_SPHERE; i++) {
+    const GEntF& e = S.entf[i];
+    const SphF f = sph_coeffs(e, o, d, dmax);
+    if (sph_reject(f, tmax)) continue;
+    if (!e.node_base && sph_upper(f) < tmax) found = i;
+    left |= 1ull << (i - first);
+  }
+  if (found >= 0) return found;
+  while (left) {
+    const int k = first + __ffsll((long long)left) - 1;
+    left &= left - 1;
+    const GEntF& e = S.entf[k];
+    const SphF f = sph_coeffs(e, o, d, dmax);
+    if (fabsf(f.c) <= f.ec && sph_reject_surface(e, f, o, tmax)) continue;
+    float t, rest;
+    if (fast_sphere(S.ents[k], o, d, tmax, t, rest)) return k;
+  }
+  return -1;
+}
+
+// ---- persistent traversal: one ray per lane, advanced step by step ---------
+enum : int { TRACE_CLOSEST = 0, TRACE_ANY = 1, TRACE_EITHER = 2 };
+
+struct TraceLane {
+  WRay ray;
+  float tmax;    // current closest (closest hit) or the ray's limit (any hit)
+  int ent;       // next entity of the list to test (the current mesh while in_mesh)
+  int sp;        // node groups on the traversal stack
+  bool in_mesh;  // inside the traversal of mesh 'ent'
+  bool any;      // TRACE_EITHER: an any-hit ray
+  WGroup g;      // the current node group
+  FastHit h;
+};
+
+__device__ __forceinline__ void lane_start(TraceLane& r, float3 o, float3 d, float tmax) {
+  r.ray = make_wray(o, d);
+  r.tmax = tmax;
+  r.ent = 0;
+  r.sp = 0;
+  r.in_mesh = false;
+  r.g.base = 0;
+  r.g.bits = 0;
+  r.h.t = tmax;
+  r.h.ent = -1;
+  r.h.slot = -1;
+  r.h.u = r.h.v = 0.0f;
+}
+
+// The bounds of a whole mesh against the ray (GEntF::u, v: the root's child
+// boxes together): a mesh missed here costs 20 instructions instead of a
+// node visit.  The bounds hold the padded root box, so no triangle is lost.
+__device__ __forceinline__ bool mesh_bounds_hit(const GEntF& e, const WRay& r, float tmax) {
+  const float x0 = (e.u[0] - r.o.x) * r.inv.x, x1 = (e.v[0] - r.o.x) * r.inv.x;
+  const float y0 = (e.u[1] - r.o.y) * r.inv.y, y1 = (e.v[1] - r.o.y) * r.inv.y;
+  const float z0 = (e.u[2] - r.o.z) * r.inv.z, z1 = (e.v[2] - r.o.z) * r.inv.z;
+  const float tn = fmax3(fminf(x0, x1), fminf(y0, y1), fmaxf(fminf(z0, z1), 0.0f));
+  const float tf = fmin3(fmaxf(x0, x1), fmaxf(y0, y1), fminf(fmaxf(z0, z1), tmax));
+  return tn <= tf;
+}
+
+// One step of a ray: the other entities up to the next mesh the ray may meet
+// (if it is not in one), then one node of that mesh with its leaf triangles
+// (fast_qbvh's loop body), so that a lane that starts a ray or a mesh shares
+// the warp's node visit.  True when the ray is answered (any hit: h.ent >= 0
+// means occluded).  Measured and not kept, within 2 % on GB300: voting per
+// step between entity, node and triangle work (16 to 20 lanes a step instead
+// of 11, paid back in votes), two triangles side by side, the next node's
+// prefetch (3 % slower).
+template <int MODE>
+__device__ __forceinline__ bool trace_step(const DevScene& S, TraceLane& r, WGroup* stack, TraceStats& st,
+                                           uint32_t* err) {
+  const bool any = MODE == TRACE_ANY || (MODE == TRACE_EITHER && r.any);
+  if (!r.in_mesh) {
+    while (r.ent < S.n_ents) {
+      const int i = r.ent;
+      const GEntF& e = S.entf[i];
+      if (e.type == PR_ENT_POLYGON) {
+        if (mesh_bounds_hit(e, r.ray, r.tmax)) {
+          r.g = wgroup_root(e.node_base, r.ray.oct);
+          r.sp = 0;
+          r.in_mesh = true;
+          break;
+        }
+        r.ent++;
+        continue;
+      }
+      if (e.type == PR_ENT_SPHERE) {
+        if (any) {
+          r.h.ent = sphere_run_any(S, r.ent, r.ray.o, r.ray.d, r.tmax);
+          if (r.h.ent >= 0) return true;
+        } else {
+          sphere_run_closest(S, r.ent, r.ray.o, r.ray.d, r.h);
+          r.tmax = r.h.t;
+        }
+        continue;
+      }
+      float t = r.tmax;
+      bool got = false;
+      if (e.type == PR_ENT_UVPLANE) got = fast_uvplane(e, r.ray.o, r.ray.d, r.tmax, t);
+      else if (e.type == PR_ENT_CIRCLE) got = fast_circle(e, r.ray.o, r.ray.d, r.tmax, t);
+      r.ent++;
+      if (any && got) {  // the test itself keeps t below the limit
+        r.h.ent = i;
+        return true;
+      }
+      if (got && t < r.tmax) {
+        r.h.ent = i;
+        r.h.slot = -1;
+        r.h.u = r.h.v = 0.0f;
+        r.tmax = t;
+        r.h.t = t;
+      }
+    }
+    if (!r.in_mesh) return true;  // past the last entity
+  }
+  if ((r.g.bits & 0xFFu) == 0) r.g = stack[--r.sp];  // stacked groups always hold a pending child
+  const int child = wgroup_next(r.g, r.ray.oct);
+  if (r.g.bits & 0xFFu) {
+    if (r.sp >= kWStack) {
+      atomicOr(err, PR_DEV_STACK_OVERFLOW);
+      return true;
+    }
+    stack[r.sp++] = r.g;
+  }
+  st.nodes++;
+  uint32_t tm;
+  int tb;
+  wnode_visit(S.rnodes + child, r.ray, r.tmax, r.g, tm, tb);
+  while (tm) {
+    const int k = __ffs(tm) - 1;
+    tm &= tm - 1u;
+    st.tris++;
+    float t, uu, vv;
+    if (fast_tri(S.rtris + 3 * (size_t)(tb + k), r.ray.o, r.ray.d, r.tmax, t, uu, vv)) {
+      r.h.ent = r.ent;
+      r.h.slot = tb + k;
+      if (any) return true;
+      r.tmax = t;
+      r.h.t = t;
+      r.h.u = uu;
+      r.h.v = vv;
+    }
+  }
+  if ((r.g.bits & 0xFFu) == 0 && r.sp == 0) {
+    r.in_mesh = false;  // this mesh is done
+    r.ent++;
+    return r.ent >= S.n_ents;
+  }
+  return false;
+}
+
 // closest hit over the entity list (strict '<' in list order)
 __device__ __forceinline__ bool fast_closest(const DevScene& S, float3 o, float3 d, FastHit& h, TraceStats& st,
                                              uint32_t* err) {
@@ -285,15 +606,18 @@ __device__ __forceinline__ bool fast_closest(const DevScene& S, float3 o, float3
   h.slot = -1;
   h.u = h.v = 0.0f;
   const WRay r = make_wray(o, d);
-  for (int i = 0; i < S.n_ents; i++) {
+  for (int i = 0; i < S.n_ents;) {
     const GEntF& e = S.entf[i];
+    if (e.type == PR_ENT_SPHERE) {
+      sphere_run_closest(S, i, o, d, h);
+      continue;
+    }
     float t = h.t, bu = 0.0f, bv = 0.0f;
     int slot = -1;
     bool got = false;
-    if (e.type == PR_ENT_SPHERE) got = fast_sphere(S.ents[i], o, d, h.t, t, bu);
-    else if (e.type == PR_ENT_UVPLANE) got = fast_uvplane(e, o, d, h.t, t);
+    if (e.type == PR_ENT_UVPLANE) got = fast_uvplane(e, o, d, h.t, t);
     else if (e.type == PR_ENT_CIRCLE) got = fast_circle(e, o, d, h.t, t);
-    else if (e.type == PR_ENT_POLYGON) got = fast_qbvh<false>(S, e, r, t, slot, bu, bv, st, err);
+    else if (e.type == PR_ENT_POLYGON && mesh_bounds_hit(e, r, h.t)) got = fast_qbvh<false>(S, e, r, t, slot, bu, bv, st, err);
     if (got && t < h.t) {
       h.t = t;
       h.ent = i;
@@ -301,6 +625,7 @@ __device__ __forceinline__ bool fast_closest(const DevScene& S, float3 o, float3
       h.u = bu;
       h.v = bv;
     }
+    i++;
   }
   return h.ent >= 0;
 }
@@ -309,16 +634,20 @@ __device__ __forceinline__ bool fast_closest(const DevScene& S, float3 o, float3
 __device__ __forceinline__ bool fast_occluded(const DevScene& S, float3 o, float3 d, float tmax, TraceStats& st,
                                               uint32_t* err) {
   const WRay r = make_wray(o, d);
-  for (int i = 0; i < S.n_ents; i++) {
+  for (int i = 0; i < S.n_ents;) {
     const GEntF& e = S.entf[i];
+    if (e.type == PR_ENT_SPHERE) {
+      if (sphere_run_any(S, i, o, d, tmax) >= 0) return true;
+      continue;
+    }
     float t = tmax, bu, bv;
     int slot;
     bool got = false;
-    if (e.type == PR_ENT_SPHERE) got = fast_sphere(S.ents[i], o, d, tmax, t, bu);
-    else if (e.type == PR_ENT_UVPLANE) got = fast_uvplane(e, o, d, tmax, t);
+    if (e.type == PR_ENT_UVPLANE) got = fast_uvplane(e, o, d, tmax, t);
     else if (e.type == PR_ENT_CIRCLE) got = fast_circle(e, o, d, tmax, t);
-    else if (e.type == PR_ENT_POLYGON) got = fast_qbvh<true>(S, e, r, t, slot, bu, bv, st, err);
+    else if (e.type == PR_ENT_POLYGON && mesh_bounds_hit(e, r, tmax)) got = fast_qbvh<true>(S, e, r, t, slot, bu, bv, st, err);
     if (got) return true;
+    i++;
   }
   return false;
 }

@@ -416,12 +416,13 @@ __global__ void __launch_bounds__(128, 6) wf_shade() { wf_shade_impl<false, fals
 // scenes with parallel, spot or infinity lights, textures or IBL images
 __global__ void __launch_bounds__(128, 4) wf_shade_ext() { wf_shade_impl<false, true>(); }
 // scenes with subsurface materials (any light kind)
-__global__ void __launch_bounds__(128, 3) wf_shade_sss() { wf_shade_impl<true, true>(); }
+// (96 registers: 3 / 4 / 5 blocks took 14.8 / 13.9 / 13.3 ms of a 320x320 x
+// 16 spp media frame with a 20,480-triangle subsurface mesh)
+__global__ void __launch_bounds__(128, 5) wf_shade_sss() { wf_shade_impl<true, true>(); }
 
 // Persistent traversal with ray replacement (Aila & Laine 2009, "Understanding
 // the efficiency of ray traversal on GPUs", dynamic ray fetch): the lanes of a
-// warp advance their rays one step at a time (the non-mesh entities of the
-// list in one step, then one mesh node with its leaves per step) and, once
+// warp advance their rays one step at a time (trace_step) and, once
 // half of the warp holds no ray, take the next queue entries with one
 // warp-aggregated atomic (half: measured on GB300 over 4 / 8 / 16 / 32 idle
 // lanes, mesh Cornell box 1024x768x64 spp: 98 / 109 / 112 / 99 Mpaths/s).  A ray visits the same nodes and triangles in the
@@ -430,106 +431,6 @@ __global__ void __launch_bounds__(128, 3) wf_shade_sss() { wf_shade_impl<true, t
 // longer idles until the longest ray of its warp is done.
 constexpr int kRefillLanes = 16;
 constexpr unsigned int kWarpStepCap = 1u << 26;
-
-struct TraceLane {
-  WRay ray;
-  float tmax;        // current closest (closest hit) or the ray's limit (any hit)
-  int ent;           // next entity of the list to test (the current mesh while in_mesh)
-  int sp;            // node groups on the traversal stack
-  bool in_mesh;      // inside the traversal of mesh 'ent'
-  WGroup g;          // the current node group
-  FastHit h;
-};
-
-__device__ __forceinline__ void lane_start(TraceLane& r, float3 o, float3 d, float tmax) {
-  r.ray = make_wray(o, d);
-  r.tmax = tmax;
-  r.ent = 0;
-  r.sp = 0;
-  r.in_mesh = false;
-  r.g.base = 0;
-  r.g.bits = 0;
-  r.h.t = tmax;
-  r.h.ent = -1;
-  r.h.slot = -1;
-  r.h.u = r.h.v = 0.0f;
-}
-
-// one step of a ray; returns true when the ray is done (ANY: r.h.ent >= 0
-// means occluded)
-template <bool ANY>
-__device__ __forceinline__ bool lane_step(const DevScene& S, TraceLane& r, WGroup* stack, TraceStats& st,
-                                          uint32_t* err) {
-  if (!r.in_mesh) {
-    // non-mesh entities up to the next mesh, in list order
-    while (r.ent < S.n_ents) {
-      const int i = r.ent;
-      const GEntF& e = S.entf[i];
-      if (e.type == PR_ENT_POLYGON) {
-        r.g = wgroup_root(e.node_base, r.ray.oct);
-        r.sp = 0;
-        r.in_mesh = true;
-        break;
-      }
-      float t = r.tmax, rest = 0.0f;
-      bool got = false;
-      if (e.type == PR_ENT_SPHERE) got = fast_sphere(S.ents[i], r.ray.o, r.ray.d, r.tmax, t, rest);
-      else if (e.type == PR_ENT_UVPLANE) got = fast_uvplane(e, r.ray.o, r.ray.d, r.tmax, t);
-      else if (e.type == PR_ENT_CIRCLE) got = fast_circle(e, r.ray.o, r.ray.d, r.tmax, t);
-      r.ent++;
-      if (ANY && got) {  // the test itself keeps t below the limit
-        r.h.ent = i;
-        return true;
-      }
-      if (got && t < r.tmax) {
-        r.h.ent = i;
-        r.h.slot = -1;
-        r.h.u = rest;  // a sphere's remainder of t (0 for planes and disks)
-        r.h.v = 0.0f;
-        r.tmax = t;
-        r.h.t = t;
-      }
-    }
-    return !r.in_mesh;  // past the last entity
-  }
-  // one node of the current mesh with its leaf triangles (fast_qbvh's loop body)
-  if ((r.g.bits & 0xFFu) == 0) r.g = stack[--r.sp];  // stacked groups always hold a pending child
-  const int child = wgroup_next(r.g, r.ray.oct);
-  if (r.g.bits & 0xFFu) {
-    if (r.sp >= kWStack) {
-      atomicOr(err, PR_DEV_STACK_OVERFLOW);
-      r.in_mesh = false;
-      r.ent = S.n_ents;
-      return true;
-    }
-    stack[r.sp++] = r.g;
-  }
-  st.nodes++;
-  uint32_t tm;
-  int tb;
-  wnode_visit(S.rnodes + child, r.ray, r.tmax, r.g, tm, tb);
-  while (tm) {
-    const int k = __ffs(tm) - 1;
-    tm &= tm - 1u;
-    st.tris++;
-    float t, uu, vv;
-    if (fast_tri(S.rtris + 3 * (size_t)(tb + k), r.ray.o, r.ray.d, r.tmax, t, uu, vv)) {
-      r.h.ent = r.ent;
-      r.h.slot = tb + k;
-      if (ANY) return true;
-      r.tmax = t;
-      r.h.t = t;
-      r.h.u = uu;
-      r.h.v = vv;
-    }
-  }
-  if ((r.g.bits & 0xFFu) == 0 && r.sp == 0) {
-    r.in_mesh = false;  // this mesh is done
-    r.ent++;
-    return r.ent >= S.n_ents;
-  }
-  return false;
-}
 
 // The persistent loop shared by wf_extend and wf_shadow.  fetch(idx, r)
 // starts queue entry idx on the lane; finish(r) stores its result.
@@ -565,7 +466,7 @@ __device__ __forceinline__ void persistent_trace(const DevScene& S, unsigned int
         }
       }
     }
-    if (busy && lane_step<ANY>(S, r, stack, st, err)) {
+    if (busy && trace_step<ANY ? TRACE_ANY : TRACE_CLOSEST>(S, r, stack, st, err)) {
       finish(r);
       busy = false;
     }
@@ -595,7 +496,7 @@ __device__ __forceinline__ void add_trace_counters(const WfBufs& B, unsigned int
 __global__ void __launch_bounds__(128, 8) wf_extend() {
   const DevScene& S = c_scene;
   const WfBufs& B = c_buf;
-  TraceStats st{0, 0};
+  TraceStats st{};
   unsigned int segs = 0;
   int slot = 0, dflag = 0;
   persistent_trace<false>(
@@ -619,7 +520,7 @@ __global__ void __launch_bounds__(128, 8) wf_extend() {
 __global__ void __launch_bounds__(128, 8) wf_shadow() {
   const DevScene& S = c_scene;
   const WfBufs& B = c_buf;
-  TraceStats st{0, 0};
+  TraceStats st{};
   unsigned int segs = 0;
   int item = 0;
   persistent_trace<true>(
