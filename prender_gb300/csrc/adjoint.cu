@@ -2,10 +2,10 @@
 // loss with respect to every material's colour (albedo) and emission.
 //
 // The caller renders the image with pr_render, forms dL/d(pixel), and calls
-// the adjoint with the same camera, parameters and sample range.  Each
-// thread replays its camera samples with the same counter-based streams, so
-// it walks exactly the paths of the forward render (Vicini, Speierer and
-// Jakob, "Path Replay Backpropagation", SIGGRAPH 2021), and accumulates:
+// the adjoint with the same camera, parameters and sample range.  The camera
+// samples are replayed with the same counter-based streams, so they walk
+// exactly the paths of the forward render (Vicini, Speierer and Jakob, "Path
+// Replay Backpropagation", SIGGRAPH 2021), and accumulate:
 //
 //  * colour: every term a branch adds to L after a non-terminal vertex j is
 //    proportional to C_{m_j} once (BRDF_Diffuse / Specular / Refraction all
@@ -25,167 +25,315 @@
 // not supported by this pass; materials are limited to kAdjMaterials.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "adjoint.h"
-#include "path_logic.cuh"
+#include "block_paths.cuh"
 
 namespace pr {
 namespace {
-
-struct Anc {
-  int8_t m[3];  // materials of the vertices before the split (depth <= 2)
-  int8_t n;
-};
 
 __device__ __forceinline__ float3 safe_div(float3 a, float3 c) {
   return f3(c.x != 0.0f ? a.x / c.x : 0.0f, c.y != 0.0f ? a.y / c.y : 0.0f, c.z != 0.0f ? a.z / c.z : 0.0f);
 }
 
-// one camera sample: returns the sample's radiance L (before the clamp) and
-// adds d L / d C_m to g_col and d L / d E_m to g_em
-__device__ float3 adjoint_sample(const DevScene& S, const RenderCfg& cfg, float3 o0, float3 d0, uint64_t sample_id,
-                                 int n_mat, float3* g_col, float3* g_em, TraceStats& st, uint32_t* err,
-                                 uint32_t& segs) {
-  PathState stack[kSplitStack];
-  Anc anc[kSplitStack];
-  int sp = 0;
-  root_path(stack[sp], o0, d0);
-  anc[sp].n = 0;
-  sp++;
-  float3 L = f3(0, 0, 0);
-  EmissionTap tap{g_em, n_mat};
-  float cnt[kAdjMaterials];
-  float3 Ssum[kAdjMaterials];
-  while (sp > 0) {
-    --sp;
-    PathState ps = stack[sp];
-    Anc mine = anc[sp];  // this branch's vertex materials so far (first three), ancestors included
-    for (int m = 0; m < n_mat; m++) {
-      cnt[m] = 0.0f;
-      Ssum[m] = f3(0, 0, 0);
-    }
-    for (int k = 0; k < mine.n; k++) cnt[mine.m[k]] += 1.0f;  // the child's radiance all comes after them
-    for (;;) {
-      FastHit h;
-      segs++;
-      const bool hit = fast_closest(S, ps.o, ps.d, h, st, err);
-      ShadowReq sh[3];
-      int nsh = 0;
-      PathState child;
-      const int r = shade<false, false>(S, cfg, ps, hit, h, sample_id, sh, nsh, child, err, nullptr, nullptr, &tap);
-      if (r != SHADE_END) {
-        // a non-terminal vertex: everything this branch adds from here on scales with its colour
-        const int m = S.entf[h.ent].material;
-        cnt[m] += 1.0f;
-        Ssum[m] += ps.L;
-        if (mine.n < 3) mine.m[mine.n++] = (int8_t)m;
-      }
-      for (int k = 0; k < nsh; k++) {
-        segs++;
-        if (!fast_occluded(S, sh[k].o, sh[k].d, sh[k].tmax, st, err)) {
-          ps.L += sh[k].contrib;
-          tap.em(sh[k].lmat, sh[k].ew);
-        }
-      }
-      if (r == SHADE_SPLIT) {
-        if (sp < kSplitStack) {
-          stack[sp] = child;
-          anc[sp] = mine;
-          sp++;
-        } else {
-          atomicOr(err, PR_DEV_LOOP_CAP);
-        }
-      }
-      if (r == SHADE_END) break;
-    }
-    for (int m = 0; m < n_mat; m++)
-      if (cnt[m] > 0.0f) g_col[m] += safe_div(ps.L * cnt[m] - Ssum[m], ld3(S.mats[m].color));
-    L += ps.L;
-  }
-  return L;
+// A pass covers whole warps of the reduction below: a warp is an 8 x 4 pixel
+// tile and a sample chunk, each lane sums its pixel's samples [k0, k1) in
+// order.  The paths themselves run in any order on resident blocks
+// (block_paths.cuh) and leave what the sums need of each sample.
+struct AdjointPass {
+  uint32_t warp0;            // first warp (chunk * tiles + tile)
+  uint32_t kk0;              // first sample of each lane in this pass
+  uint32_t kmax;             // samples of each lane in this pass
+  int first, last;           // of the passes over these lanes' samples
+  unsigned long long items;  // warps * 32 * kmax (sample kk of lane l of warp w: (w 32 + l) kmax + kk)
+  unsigned long long* next;  // items handed out
+  int n_mat;
+  float3* w;                 // per item: dLoss / d(sample radiance); zero where there is no sample
+  float3* g_col;             // per item and material: d L / d C_m
+  float3* g_em;              // d L / d E_m
+  float4* acc;               // per slot and material: sum S_m of the branch, count n_m
+  int* anc;                  // per slot: materials of the branch's first three vertices, their number << 24
+  unsigned long long* item;  // per slot
+  float4* ew;                // 3 per slot: contribution / emission of the queued shadow rays
+  float* carry;              // 6 per lane and material: sums carried to the lanes' next pass
+};
+
+// pixel and sample of an item; false where the tile or the chunk has none
+__device__ __forceinline__ bool adjoint_item(const RenderCfg& cfg, const AdjointPass& A, unsigned long long it, int& x,
+                                             int& y, int& k) {
+  const uint32_t v = (uint32_t)(it / A.kmax), kk = (uint32_t)(it - (unsigned long long)v * A.kmax);
+  const uint32_t warp = A.warp0 + (v >> 5), lane = v & 31;
+  const uint32_t tiles = cfg.tiles_x * cfg.tiles_y, chunk = warp / tiles, tile = warp - chunk * tiles;
+  x = (int)((tile % cfg.tiles_x) * 8 + (lane & 7));
+  y = (int)((tile / cfg.tiles_x) * 4 + (lane >> 3));
+  const int k0 = (int)(((int64_t)cfg.spp * chunk) / cfg.chunks);
+  const int k1 = (int)(((int64_t)cfg.spp * (chunk + 1)) / cfg.chunks);
+  k = k0 + (int)(A.kk0 + kk);
+  return x < cfg.width && y < cfg.height && k < k1;
 }
 
-}  // namespace
+struct AdjointPaths {
+  const DevScene& S;
+  const RenderCfg& cfg;
+  const AdjointPass& A;
+  const BlockPool& P;
+  const float* dl_drgb;
+  uint32_t* err;
+  uint32_t paths;
+  bool more;
 
-__global__ void __launch_bounds__(128) adjoint_kernel(DevScene S, RenderCfg cfg, const float* __restrict__ dl_drgb,
-                                                      int n_mat, double* __restrict__ d_color,
-                                                      double* __restrict__ d_emission, uint32_t* __restrict__ err,
-                                                      unsigned long long* __restrict__ counters) {
-  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t warp = tid >> 5, lane = tid & 31;
-  const uint32_t tiles_per_chunk = cfg.tiles_x * cfg.tiles_y;
-  const uint32_t chunk = warp / tiles_per_chunk;
-  if (chunk >= (uint32_t)cfg.chunks) return;  // whole warps leave together
-  const uint32_t tile = warp - chunk * tiles_per_chunk;
-  const int x = (int)((tile % cfg.tiles_x) * 8 + (lane & 7));
-  const int y = (int)((tile / cfg.tiles_x) * 4 + (lane >> 3));
-  float3 G_col[kAdjMaterials], G_em[kAdjMaterials];
-  for (int m = 0; m < kAdjMaterials; m++) G_col[m] = G_em[m] = f3(0, 0, 0);
-  TraceStats st{0, 0};
-  uint32_t segs = 0, paths = 0;
-  if (x < cfg.width && y < cfg.height) {
-    const size_t pix = (size_t)(cfg.height - y - 1) * cfg.width + x;
-    const float3 delta = f3(dl_drgb[3 * pix], dl_drgb[3 * pix + 1], dl_drgb[3 * pix + 2]) * cfg.sensor;
-    const int k0 = (int)(((int64_t)cfg.spp * chunk) / cfg.chunks);
-    const int k1 = (int)(((int64_t)cfg.spp * (chunk + 1)) / cfg.chunks);
-    float3 g_col[kAdjMaterials], g_em[kAdjMaterials];
-    for (int k = k0; k < k1; k++) {
-      for (int m = 0; m < n_mat; m++) g_col[m] = g_em[m] = f3(0, 0, 0);
+  __device__ __forceinline__ void start_branch(size_t i, int anc) {
+    float4* acc = A.acc + i * A.n_mat;
+    for (int m = 0; m < A.n_mat; m++) acc[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    // the branch's radiance all comes after its ancestors' vertices
+    for (int k = 0; k < (anc >> 24); k++) acc[(anc >> (8 * k)) & 0xFF].w += 1.0f;
+    A.anc[i] = anc;
+  }
+
+  __device__ __forceinline__ bool take(bool want, size_t i, PathState& ps) {
+    const int lane = threadIdx.x & 31;
+    bool got = false;
+    for (;;) {
+      const unsigned int mask = __ballot_sync(0xffffffffu, want && !got && more);
+      if (!mask) return got;
+      unsigned long long base = 0;
+      const int leader = __ffs(mask) - 1;
+      if (lane == leader) base = atomicAdd(A.next, (unsigned long long)__popc(mask));
+      base = __shfl_sync(0xffffffffu, base, leader);
+      if (!((mask >> lane) & 1)) continue;
+      const unsigned long long it = base + (unsigned long long)__popc(mask & ((1u << lane) - 1u));
+      if (it >= A.items) {
+        more = false;
+        continue;
+      }
+      int x, y, k;
+      if (!adjoint_item(cfg, A, it, x, y, k)) continue;
       float3 o, d;
-      const uint64_t sample_id = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
-      const float3 L = adjoint_sample(S, cfg, o, d, sample_id, n_mat, g_col, g_em, st, err, segs);
-      // finish_sample: v = L * smp, and above the cutoff v_c = c v / lum(v),
-      // whose derivative is (c / lum) (dv - v (W . dv) / lum) with W the
-      // luminance weights: the adjoint of the clamp maps delta to
-      // (c / lum) (delta - (delta . v / lum) W)
-      const float3 v = L * cfg.smp;
-      float3 w = delta * cfg.smp;
-      if (!(isfinite(v.x) && isfinite(v.y) && isfinite(v.z))) {
-        w = f3(0, 0, 0);
-      } else if (cfg.cutoff > 0.0f) {
-        const float3 W = f3(0.2126f, 0.7152f, 0.0722f);
-        const float lum = dot(W, v);
-        if (lum > cfg.cutoff) w = (delta - W * (dot(delta, v) / lum)) * (cfg.cutoff / lum * cfg.smp);
-      }
-      for (int m = 0; m < n_mat; m++) {
-        G_col[m] += w * g_col[m];
-        G_em[m] += w * g_em[m];
-      }
-      paths++;
+      P.id[i] = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
+      root_path(ps, o, d);
+      A.item[i] = it;
+      start_branch(i, 0);
+      got = true;
     }
   }
-  // warp sums, then one double atomic per value and warp
-  for (int m = 0; m < n_mat; m++) {
-    float v[6] = {G_col[m].x, G_col[m].y, G_col[m].z, G_em[m].x, G_em[m].y, G_em[m].z};
+
+  __device__ __forceinline__ EmissionTap tap(size_t i) const { return EmissionTap{A.g_em + A.item[i] * A.n_mat, A.n_mat}; }
+
+  __device__ __forceinline__ void nee(size_t i, PathState& ps, int n, const unsigned char* lit) {
+    EmissionTap t = tap(i);
+    for (int k = 0; k < 3; k++)
+      if (k < n && lit[k]) {
+        const float4 c = P.sh_c[3 * i + k], e = A.ew[3 * i + k];
+        ps.L += f3(c.x, c.y, c.z);
+        t.em(__float_as_int(c.w), f3(e.x, e.y, e.z));
+      }
+  }
+  __device__ __forceinline__ void queued(size_t i, int k, const ShadowReq& r) {
+    A.ew[3 * i + k] = make_float4(r.ew.x, r.ew.y, r.ew.z, 0.0f);
+  }
+
+  __device__ __forceinline__ int vertex(size_t i, PathState& ps, int& pending, bool hit, const FastHit& h,
+                                        ShadowReq* sh, int& nsh) {
+    PathState child;
+    const unsigned long long id = P.id[i];
+    EmissionTap t = tap(i);
+    const int r = shade<false, false>(S, cfg, ps, hit, h, id, sh, nsh, child, err, nullptr, nullptr, &t);
+    int anc = A.anc[i];
+    if (r != SHADE_END) {
+      // a non-terminal vertex: everything this branch adds from here on scales with its colour
+      const int m = S.entf[h.ent].material;
+      float4& a = A.acc[i * A.n_mat + m];
+      a.w += 1.0f;
+      a.x += ps.L.x;
+      a.y += ps.L.y;
+      a.z += ps.L.z;
+      if ((anc >> 24) < 3) {
+        anc = (anc & 0xFFFFFF) | (m << (8 * (anc >> 24))) | (((anc >> 24) + 1) << 24);
+        A.anc[i] = anc;
+      }
+    }
+    if (r == SHADE_SPLIT) {
+      const int n = pending & 0xFF;
+      if (n < kSplitStack) {
+        block_push(P, i, n, child, anc);
+        if (!(pending & 0x100)) P.root[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        pending = (n + 1) | 0x100;
+      } else {
+        atomicOr(err, PR_DEV_LOOP_CAP);
+      }
+    }
+    if (r != SHADE_END) return r;
+    nsh = 0;
+    const unsigned long long it = A.item[i];
+    for (int m = 0; m < A.n_mat; m++) {
+      const float4 a = A.acc[i * A.n_mat + m];
+      if (a.w > 0.0f)
+        A.g_col[it * A.n_mat + m] += safe_div(ps.L * a.w - f3(a.x, a.y, a.z), ld3(S.mats[m].color));
+    }
+    float3 L = ps.L;
+    if (pending & 0x100) {
+      const float4 q = P.root[i];
+      L = f3(q.x, q.y, q.z) + ps.L;
+      const int n = pending & 0xFF;
+      if (n > 0) {  // the next branch that waits
+        P.root[i] = make_float4(L.x, L.y, L.z, 0.0f);
+        start_branch(i, block_pop(P, i, n - 1, ps));
+        pending--;
+        return SHADE_CONTINUE;
+      }
+    }
+    // finish_sample: v = L * smp, and above the cutoff v_c = c v / lum(v),
+    // whose derivative is (c / lum) (dv - v (W . dv) / lum) with W the
+    // luminance weights: the adjoint of the clamp maps delta to
+    // (c / lum) (delta - (delta . v / lum) W)
+    int x, y, k;
+    adjoint_item(cfg, A, it, x, y, k);
+    const size_t pix = (size_t)(cfg.height - y - 1) * cfg.width + x;
+    const float3 delta = f3(dl_drgb[3 * pix], dl_drgb[3 * pix + 1], dl_drgb[3 * pix + 2]) * cfg.sensor;
+    const float3 v = L * cfg.smp;
+    float3 w = delta * cfg.smp;
+    if (!(isfinite(v.x) && isfinite(v.y) && isfinite(v.z))) {
+      w = f3(0, 0, 0);
+    } else if (cfg.cutoff > 0.0f) {
+      const float3 W = f3(0.2126f, 0.7152f, 0.0722f);
+      const float lum = dot(W, v);
+      if (lum > cfg.cutoff) w = (delta - W * (dot(delta, v) / lum)) * (cfg.cutoff / lum * cfg.smp);
+    }
+    A.w[it] = w;
+    paths++;
+    return SHADE_END;
+  }
+};
+
+__global__ void __launch_bounds__(kBlockThreads, 1)
+    adjoint_paths(const __grid_constant__ DevScene S, const __grid_constant__ RenderCfg cfg,
+                  const __grid_constant__ AdjointPass A, const __grid_constant__ BlockPool P,
+                  const float* __restrict__ dl_drgb, uint32_t* __restrict__ err,
+                  unsigned long long* __restrict__ counters) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  TraceStats st{0, 0};
+  uint32_t segs = 0;
+  AdjointPaths drv{S, cfg, A, P, dl_drgb, err, 0u, true};
+  block_paths(S, P, drv, smem, st, segs, err);
+  if (counters) add_counters(counters, drv.paths, segs, st);
+}
+
+// the samples' gradients of a pass: each lane its pixel's samples in order,
+// then the warp, then one double atomic per value and warp
+__global__ void __launch_bounds__(128) adjoint_reduce(const __grid_constant__ AdjointPass A, double* __restrict__ d_color,
+                                                      double* __restrict__ d_emission) {
+  const unsigned long long v = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if ((v >> 5) * 32ull * A.kmax >= A.items) return;  // whole warps leave together
+  const int lane = threadIdx.x & 31;
+  for (int m = 0; m < A.n_mat; m++) {
+    float3 col = f3(0, 0, 0), em = f3(0, 0, 0);
+    float* c = A.carry + 6 * (v * A.n_mat + m);
+    if (!A.first) {
+      col = f3(c[0], c[1], c[2]);
+      em = f3(c[3], c[4], c[5]);
+    }
+    for (uint32_t k = 0; k < A.kmax; k++) {
+      const unsigned long long it = v * A.kmax + k;
+      const float3 w = A.w[it];
+      col += w * A.g_col[it * A.n_mat + m];
+      em += w * A.g_em[it * A.n_mat + m];
+    }
+    if (!A.last) {
+      c[0] = col.x;
+      c[1] = col.y;
+      c[2] = col.z;
+      c[3] = em.x;
+      c[4] = em.y;
+      c[5] = em.z;
+      continue;
+    }
+    const float q6[6] = {col.x, col.y, col.z, em.x, em.y, em.z};
 #pragma unroll
     for (int q = 0; q < 6; q++) {
-      float a = v[q];
+      float a = q6[q];
       for (int off = 16; off > 0; off >>= 1) a += __shfl_down_sync(0xffffffffu, a, off);
       if (lane == 0 && a != 0.0f) atomicAdd((q < 3 ? d_color : d_emission) + 3 * m + (q % 3), (double)a);
     }
   }
-  if (counters) {
-    unsigned long long a = paths, b = segs, c = st.nodes, dd = st.tris;
-    for (int off = 16; off > 0; off >>= 1) {
-      a += __shfl_down_sync(0xffffffffu, a, off);
-      b += __shfl_down_sync(0xffffffffu, b, off);
-      c += __shfl_down_sync(0xffffffffu, c, off);
-      dd += __shfl_down_sync(0xffffffffu, dd, off);
-    }
-    if (lane == 0) {
-      atomicAdd(counters + 0, a);
-      atomicAdd(counters + 1, b);
-      atomicAdd(counters + 2, c);
-      atomicAdd(counters + 3, dd);
-    }
-  }
 }
 
-cudaError_t launch_adjoint(const DevScene& S, const RenderCfg& cfg, const float* dl_drgb, int n_mat, double* d_color,
-                           double* d_emission, uint32_t* err, unsigned long long* counters, cudaStream_t stream) {
-  const uint64_t threads = (uint64_t)cfg.tiles_x * cfg.tiles_y * 32ull * (uint64_t)cfg.chunks;
-  const uint32_t blocks = (uint32_t)((threads + 127) / 128);
-  adjoint_kernel<<<blocks, 128, 0, stream>>>(S, cfg, dl_drgb, n_mat, d_color, d_emission, err, counters);
-  return cudaGetLastError();
+constexpr size_t kAdjointBytes = 512ull << 20;  // of the samples of one pass (a lane's at most kAdjointLane)
+constexpr uint32_t kAdjointLane = 4096;
+
+// warps and samples per lane of a pass, and the scratch it takes
+struct AdjointShape {
+  uint32_t warps, pass_warps, lane_samples, kmax;  // kmax: a lane's samples in one pass
+  size_t item_bytes, slot_bytes, slots, carry_bytes;
+};
+AdjointShape adjoint_shape(const RenderCfg& cfg, int n_mat) {
+  AdjointShape h;
+  h.warps = cfg.tiles_x * cfg.tiles_y * (uint32_t)cfg.chunks;
+  h.lane_samples = (uint32_t)((cfg.spp + cfg.chunks - 1) / cfg.chunks);
+  h.kmax = std::min(h.lane_samples, kAdjointLane);
+  h.item_bytes = sizeof(float3) * (1 + 2 * (size_t)n_mat);
+  const size_t per_warp = h.item_bytes * 32 * h.kmax;
+  h.pass_warps = (uint32_t)std::max<size_t>(1, std::min<size_t>(h.warps, kAdjointBytes / per_warp));
+  const BlockShape b = block_shape((unsigned long long)h.pass_warps * 32 * h.kmax, sm_count());
+  h.slots = (size_t)b.blocks * b.slots;
+  h.slot_bytes = sizeof(float4) * (n_mat + 3) + 4 + 8;
+  h.carry_bytes = h.lane_samples > h.kmax ? 24 * (size_t)n_mat * 32 * h.pass_warps : 0;
+  return h;
+}
+
+}  // namespace
+
+size_t adjoint_scratch_bytes(const RenderCfg& cfg, int n_mat) {
+  const AdjointShape h = adjoint_shape(cfg, n_mat);
+  return 256 + (h.item_bytes * h.pass_warps * 32 * h.kmax + 255) / 256 * 256 + block_pool_bytes(h.slots) +
+         (h.slot_bytes * h.slots + 255) / 256 * 256 + h.carry_bytes + 256;
+}
+
+cudaError_t launch_adjoint(const DevScene& S, const RenderCfg& cfg, const float* dl_drgb, int n_mat, void* scratch,
+                           double* d_color, double* d_emission, uint32_t* err, unsigned long long* counters,
+                           int* launches, cudaStream_t stream) {
+  const AdjointShape h = adjoint_shape(cfg, n_mat);
+  *launches = 0;
+  for (uint32_t w0 = 0; w0 < h.warps; w0 += h.pass_warps)
+    for (uint32_t k0 = 0; k0 < h.lane_samples; k0 += h.kmax) {
+      const uint32_t warps = std::min(h.pass_warps, h.warps - w0);
+      AdjointPass A;
+      A.warp0 = w0;
+      A.kk0 = k0;
+      A.kmax = std::min(h.kmax, h.lane_samples - k0);
+      A.first = k0 == 0;
+      A.last = k0 + A.kmax == h.lane_samples;
+      A.items = (unsigned long long)warps * 32 * A.kmax;
+      A.n_mat = n_mat;
+      char* p = static_cast<char*>(scratch);
+      A.next = reinterpret_cast<unsigned long long*>(p);
+      A.w = reinterpret_cast<float3*>(p + 256);
+      A.g_col = A.w + A.items;
+      A.g_em = A.g_col + A.items * n_mat;
+      const size_t zero = 256 + h.item_bytes * A.items;
+      cudaError_t e = cudaMemsetAsync(p, 0, zero, stream);
+      if (e != cudaSuccess) return e;
+      p += (zero + 255) / 256 * 256;
+      const BlockShape b = block_shape(A.items, sm_count());
+      const size_t n = (size_t)b.blocks * b.slots;
+      BlockPool P = block_pool(p, n);
+      P.slots = b.slots;
+      P.slots_used = b.used;
+      p += (block_pool_bytes(n) + 255) / 256 * 256;
+      A.acc = reinterpret_cast<float4*>(p);
+      A.ew = A.acc + n * n_mat;
+      A.item = reinterpret_cast<unsigned long long*>(A.ew + 3 * n);
+      A.anc = reinterpret_cast<int*>(A.item + n);
+      A.carry = reinterpret_cast<float*>(p + (h.slot_bytes * n + 255) / 256 * 256);
+      adjoint_paths<<<b.blocks, b.threads, block_shared_bytes(b.slots), stream>>>(S, cfg, A, P, dl_drgb, err, counters);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+      adjoint_reduce<<<(warps + 3) / 4, 128, 0, stream>>>(A, d_color, d_emission);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+      *launches += 2;
+    }
+  return cudaSuccess;
 }
 
 }  // namespace pr

@@ -10,8 +10,11 @@ namespace pr {
 constexpr int kAdjMaterials = 16;  // materials the adjoint pass tracks
 
 // adds dL/dC (3 per material) and dL/dE (3 per material) into d_color and
-// d_emission (device, double); same launch geometry as the megakernel
-cudaError_t launch_adjoint(const DevScene& S, const RenderCfg& cfg, const float* dl_drgb, int n_mat, double* d_color,
-                           double* d_emission, uint32_t* err, unsigned long long* counters, cudaStream_t stream);
+// d_emission (device, double); scratch of adjoint_scratch_bytes; launches:
+// the kernels launched
+size_t adjoint_scratch_bytes(const RenderCfg& cfg, int n_mat);
+cudaError_t launch_adjoint(const DevScene& S, const RenderCfg& cfg, const float* dl_drgb, int n_mat, void* scratch,
+                           double* d_color, double* d_emission, uint32_t* err, unsigned long long* counters,
+                           int* launches, cudaStream_t stream);
 
 }  // namespace pr

@@ -109,7 +109,7 @@ void pr_destroy(pr_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   c->cur.release();
   for (DevBuf* b : {&c->k_status, &c->k_bl, &c->k_dir, &c->k_steps, &c->k_ent, &c->k_t,
-                    &c->adj_scratch, &c->adj_grad, &c->k_sens})
+                    &c->adj_scratch, &c->adj_grad, &c->adj_samples, &c->k_sens})
     b->release();
   for (DevBuf* b : {&c->errword, &c->counters, &c->partial,
                     &c->out, &c->rays, &c->ires, &c->jres, &c->dres, &c->wf_o, &c->wf_d, &c->wf_beta, &c->wf_dpw,
@@ -1009,18 +1009,20 @@ int pr_render_adjoint_dev(pr_ctx* c, const pr_camera* cam, const pr_render_param
   double* de = d_emission ? d_emission : (double*)c->adj_scratch.p + 3 * std::max(n_mat, 1);
   if (!d_color) PR_CUDA(c, cudaMemsetAsync(dc, 0, 3 * sizeof(double) * n_mat, c->stream));
   if (!d_emission) PR_CUDA(c, cudaMemsetAsync(de, 0, 3 * sizeof(double) * n_mat, c->stream));
+  PR_CUDA(c, c->adj_samples.ensure(adjoint_scratch_bytes(g, n_mat)));
   PR_CUDA(c, cudaMemsetAsync(c->errword.p, 0, 4, c->stream));
   PR_CUDA(c, cudaMemsetAsync(c->counters.p, 0, 128, c->stream));
   PR_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-  PR_CUDA(c, launch_adjoint(c->cur.dev, g, dl_drgb, n_mat, dc, de, (uint32_t*)c->errword.p,
-                            (unsigned long long*)c->counters.p, c->stream));
+  int launches = 0;
+  PR_CUDA(c, launch_adjoint(c->cur.dev, g, dl_drgb, n_mat, c->adj_samples.p, dc, de, (uint32_t*)c->errword.p,
+                            (unsigned long long*)c->counters.p, &launches, c->stream));
   PR_CUDA(c, cudaEventRecord(c->ev1, c->stream));
   unsigned long long cnt[16];
   PR_CUDA(c, cudaMemcpyAsync(cnt, c->counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, c->stream));
   st = check_device_errors(c);
   float ms = 0;
   cudaEventElapsedTime(&ms, c->ev0, c->ev1);
-  c->stats = pr_render_stats{cnt[0], cnt[1], cnt[2], cnt[3], ms, 1};
+  c->stats = pr_render_stats{cnt[0], cnt[1], cnt[2], cnt[3], ms, (uint64_t)launches};
   return st;
 }
 

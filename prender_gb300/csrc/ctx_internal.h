@@ -66,6 +66,7 @@ struct pr_ctx {
   pr::DevBuf k_sens;                                        // pr_kerr_sensitivity staging
   pr::DevBuf mlt_lum, mlt_path, mlt_start, mlt_u, mlt_cur, mlt_acc;  // PR_MODE_MLT state
   pr::DevBuf adj_scratch, adj_grad;                         // adjoint outputs
+  pr::DevBuf adj_samples;                                   // a pass's samples and path slots
   double kernel_ms[4] = {0, 0, 0, 0};        // wavefront shade / extend / shadow / control (host-driven loop)
   unsigned long long shadow_counts[3] = {0, 0, 0};  // shadow rays, nodes, triangles of the last wavefront frame
   pr_render_stats stats{};
