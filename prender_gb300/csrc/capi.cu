@@ -925,6 +925,10 @@ int pr_render_dev(pr_ctx* c, const pr_camera* cam, const pr_render_params* p, fl
   } else if (p->mode == PR_MODE_WAVEFRONT) {
     st = render_wavefront(c, g, rgb_dev, accumulate);
     if (st != PR_OK) return st;
+  } else if (!c->cur.dev.has_sss) {
+    PR_CUDA(c, c->partial.ensure(plain_scratch_bytes(g)));
+    PR_CUDA(c, launch_plain(c->cur.dev, g, c->partial.p, rgb_dev, accumulate, (uint32_t*)c->errword.p,
+                             (unsigned long long*)c->counters.p, c->stream));
   } else {
     PR_CUDA(c, c->partial.ensure(sizeof(float) * n3 * (size_t)g.chunks));
     PR_CUDA(c, launch_megakernel(c->cur.dev, g, (float*)c->partial.p, (uint32_t*)c->errword.p,
@@ -1406,6 +1410,9 @@ int pr_kerr_sensitivity_adjoint(pr_ctx* c, const double* rays, int64_t n, const 
   return kerr_sens_common(c, rays, n, basis, cotangent, nullptr, nullptr, nullptr, grad);
 }
 
+// the plain form of this scene is the stream kernel (straight rays, no subsurface materials)
+static bool streamed(const SceneObjData& sc) { return !sc.kerr.enabled && !sc.worm.enabled && !sc.dev.has_sss; }
+
 // Many jobs (scene object, camera, parameters, output) as one captured CUDA
 // graph: each job is the megakernel form (one render kernel + the ordered
 // chunk reduction) on its own branch of the graph, so small and large
@@ -1433,7 +1440,11 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
     // the batch fills the GPU with many jobs: fewer sample chunks per job
     cfg[j].chunks = std::max(1, std::min(cfg[j].chunks, (int)std::ceil(2.0e5 / ((double)cfg[j].width * cfg[j].height))));
     cfg[j].chunks = std::min(cfg[j].chunks, cfg[j].spp);
-    off[j + 1] = off[j] + (size_t)cfg[j].width * cfg[j].height * 3 * (size_t)cfg[j].chunks;
+    const SceneObjData& sc = J.scene->data;
+    size_t bytes = sizeof(float) * (size_t)cfg[j].width * cfg[j].height * 3 * (size_t)cfg[j].chunks;
+    if (J.params.mode == PR_MODE_WAVEFRONT && !sc.kerr.enabled && !sc.worm.enabled) bytes = 0;
+    else if (streamed(sc)) bytes = plain_scratch_bytes(cfg[j]);
+    off[j + 1] = off[j] + (bytes + 255) / 256 * 256;
     paths += (uint64_t)cfg[j].spp * cfg[j].width * cfg[j].height;
   }
   // jobs in the wavefront form share the context's path pool: they run one
@@ -1442,7 +1453,7 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
   for (int j = 0; j < n; j++)
     wf_job[j] = jobs[j].params.mode == PR_MODE_WAVEFRONT && !jobs[j].scene->data.kerr.enabled &&
                 !jobs[j].scene->data.worm.enabled;
-  PR_CUDA(c, c->batch_partial.ensure(sizeof(float) * std::max<size_t>(off[n], 1)));
+  PR_CUDA(c, c->batch_partial.ensure(std::max<size_t>(off[n], 1)));
   const int n_streams = std::min(n, 16);
   while ((int)c->batch_streams.size() < n_streams) {
     cudaStream_t st;
@@ -1462,23 +1473,29 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
   cudaError_t e = cudaEventRecord(c->batch_events[n_streams], c->stream);
   for (int k = 0; k < n_streams && e == cudaSuccess; k++)
     e = cudaStreamWaitEvent(c->batch_streams[k], c->batch_events[n_streams], 0);
-  float* part = (float*)c->batch_partial.p;
+  char* part = (char*)c->batch_partial.p;
   for (int j = 0; j < n && e == cudaSuccess; j++) {
     if (wf_job[j]) continue;
     const pr_job& J = jobs[j];
     cudaStream_t st = c->batch_streams[j % n_streams];
     const SceneObjData& sc = J.scene->data;
     const int n3 = cfg[j].width * cfg[j].height * 3;
+    float* partial = (float*)(part + off[j]);
+    if (streamed(sc)) {
+      e = launch_plain(sc.dev, cfg[j], partial, J.rgb_dev, J.accumulate, (uint32_t*)c->errword.p,
+                        (unsigned long long*)c->counters.p, st);
+      continue;
+    }
     if (sc.kerr.enabled)
-      e = launch_kerr_render(sc.dev, sc.kerr, cfg[j], part + off[j], (uint32_t*)c->errword.p,
+      e = launch_kerr_render(sc.dev, sc.kerr, cfg[j], partial, (uint32_t*)c->errword.p,
                              (unsigned long long*)c->counters.p, st);
     else if (sc.worm.enabled)
-      e = launch_worm_render(sc.dev, sc.worm, cfg[j], part + off[j], (uint32_t*)c->errword.p,
+      e = launch_worm_render(sc.dev, sc.worm, cfg[j], partial, (uint32_t*)c->errword.p,
                              (unsigned long long*)c->counters.p, st);
     else
-      e = launch_megakernel(sc.dev, cfg[j], part + off[j], (uint32_t*)c->errword.p,
+      e = launch_megakernel(sc.dev, cfg[j], partial, (uint32_t*)c->errword.p,
                             (unsigned long long*)c->counters.p, st);
-    if (e == cudaSuccess) e = launch_reduce(part + off[j], J.rgb_dev, n3, cfg[j].chunks, J.accumulate, st);
+    if (e == cudaSuccess) e = launch_reduce(partial, J.rgb_dev, n3, cfg[j].chunks, J.accumulate, st);
   }
   for (int k = 0; k < n_streams && e == cudaSuccess; k++) {
     e = cudaEventRecord(c->batch_events[k], c->batch_streams[k]);

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include "path_logic.cuh"
+#include "block_paths.cuh"
 
 namespace pr {
 
@@ -162,22 +163,7 @@ __global__ void __launch_bounds__(128, SSS ? 3 : 8) pt_megakernel(DevScene S, Re
     o[1] = acc.y;
     o[2] = acc.z;
   }
-  if (counters) {
-    // warp-reduced statistics
-    unsigned long long a = paths, b2 = segs, c = st.nodes, dd = st.tris;
-    for (int off = 16; off > 0; off >>= 1) {
-      a += __shfl_down_sync(0xffffffffu, a, off);
-      b2 += __shfl_down_sync(0xffffffffu, b2, off);
-      c += __shfl_down_sync(0xffffffffu, c, off);
-      dd += __shfl_down_sync(0xffffffffu, dd, off);
-    }
-    if (lane == 0) {
-      atomicAdd(counters + 0, a);
-      atomicAdd(counters + 1, b2);
-      atomicAdd(counters + 2, c);
-      atomicAdd(counters + 3, dd);
-    }
-  }
+  if (counters) add_counters(counters, paths, segs, st);
 }
 
 // sums the per-chunk partial images in chunk order (deterministic) into
@@ -189,6 +175,168 @@ __global__ void reduce_chunks(const float* __restrict__ partial, float* __restri
   float s = accumulate ? dst[i] : 0.0f;
   for (int c = 0; c < chunks; c++) s += partial[(size_t)c * n3 + i];
   dst[i] = s;
+}
+
+// ---- the plain form without subsurface frames ------------------------------
+// Resident blocks take camera samples one by one, pixel by pixel
+// (block_paths.cuh), and add each finished sample to its pixel in 64-bit
+// fixed point (2^-40: integer sums do not depend on the order in which
+// samples finish).
+constexpr float kPixelScaleF = 1099511627776.0f;  // 2^40
+constexpr float kPixelInvF = 1.0f / 1099511627776.0f;
+
+struct PlainFrame {
+  long long* pix;              // 3 per pixel
+  unsigned long long* next;    // samples handed out
+  unsigned long long samples;  // of the frame
+};
+
+template <bool FULL>
+struct PlainPaths {
+  const DevScene& S;
+  const RenderCfg& cfg;
+  const PlainFrame& F;
+  const BlockPool& P;
+  uint32_t* err;
+  uint32_t paths;
+  bool more;
+
+  __device__ __forceinline__ bool take(bool want, size_t i, PathState& ps) {
+    const int lane = threadIdx.x & 31;
+    const unsigned int mask = __ballot_sync(0xffffffffu, want && more);
+    if (!mask) return false;
+    unsigned long long base = 0;
+    const int leader = __ffs(mask) - 1;
+    if (lane == leader) base = atomicAdd(F.next, (unsigned long long)__popc(mask));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (!((mask >> lane) & 1)) return false;
+    const unsigned long long g = base + (unsigned long long)__popc(mask & ((1u << lane) - 1u));
+    if (g >= F.samples) {
+      more = false;
+      return false;
+    }
+    // a pixel's samples one after another: the first segments of a warp are close together
+    const unsigned long long px = g / (unsigned int)cfg.spp;
+    const uint32_t k = (uint32_t)(g - px * (unsigned int)cfg.spp);
+    const int y = (int)((uint32_t)px / (uint32_t)cfg.width), x = (int)((uint32_t)px - (uint32_t)y * cfg.width);
+    float3 o, d;
+    P.id[i] = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
+    root_path(ps, o, d);
+    return true;
+  }
+
+  __device__ __forceinline__ void nee(size_t i, PathState& ps, int n, const unsigned char* lit) {
+    float3 sum = f3(0, 0, 0);
+    for (int k = 0; k < 3; k++)
+      if (k < n && lit[k]) {
+        const float4 c = P.sh_c[3 * i + k];
+        sum += f3(c.x, c.y, c.z);
+      }
+    ps.L += sum;
+  }
+  __device__ __forceinline__ void queued(size_t, int, const ShadowReq&) {}
+
+  __device__ __forceinline__ int vertex(size_t i, PathState& ps, int& pending, bool hit, const FastHit& h,
+                                        ShadowReq* sh, int& nsh) {
+    PathState child;
+    const unsigned long long id = P.id[i];
+    // FULL: the per-thread form's fuller instantiation itself (its subsurface
+    // case is not reached), so that both round alike
+    SssFrameOut fo;
+    fo.open = 0;
+    const int r = shade<FULL, FULL, FULL>(S, cfg, ps, hit, h, id, sh, nsh, child, err, nullptr, nullptr, nullptr,
+                                          FULL ? &fo : nullptr);
+    // pending: waiting branches; bit 8: the sample has split
+    if (r == SHADE_SPLIT) {
+      const int n = pending & 0xFF;
+      if (n < kSplitStack) {
+        block_push(P, i, n, child, 0);
+        if (!(pending & 0x100)) P.root[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        pending = (n + 1) | 0x100;
+      } else {
+        atomicOr(err, PR_DEV_LOOP_CAP);
+      }
+    }
+    if (r != SHADE_END) return r;
+    nsh = 0;
+    float3 L = ps.L;
+    if (pending & 0x100) {
+      const float4 q = P.root[i];
+      L = f3(q.x, q.y, q.z) + ps.L;
+      const int n = pending & 0xFF;
+      if (n > 0) {  // the next branch that waits
+        P.root[i] = make_float4(L.x, L.y, L.z, 0.0f);
+        block_pop(P, i, n - 1, ps);
+        pending--;
+        return SHADE_CONTINUE;
+      }
+    }
+    const float3 v = finish_sample(cfg, L, err);
+    const uint32_t p = (uint32_t)(id % ((unsigned long long)cfg.width * cfg.height));
+    const uint32_t y = p / (uint32_t)cfg.width, x = p - y * (uint32_t)cfg.width;
+    unsigned long long* px =
+        reinterpret_cast<unsigned long long*>(F.pix + 3 * ((size_t)(cfg.height - 1 - y) * cfg.width + x));
+    atomicAdd(px + 0, (unsigned long long)__float2ll_rn(v.x * kPixelScaleF));
+    atomicAdd(px + 1, (unsigned long long)__float2ll_rn(v.y * kPixelScaleF));
+    atomicAdd(px + 2, (unsigned long long)__float2ll_rn(v.z * kPixelScaleF));
+    paths++;
+    return SHADE_END;
+  }
+};
+
+template <bool FULL>
+__global__ void __launch_bounds__(kBlockThreads, 1)
+    pt_block(const __grid_constant__ DevScene S, const __grid_constant__ RenderCfg cfg,
+             const __grid_constant__ PlainFrame F, const __grid_constant__ BlockPool P, uint32_t* __restrict__ err,
+             unsigned long long* __restrict__ counters) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  TraceStats st{0, 0};
+  uint32_t segs = 0;
+  PlainPaths<FULL> drv{S, cfg, F, P, err, 0u, true};
+  block_paths(S, P, drv, smem, st, segs, err);
+  if (counters) add_counters(counters, drv.paths, segs, st);
+}
+
+// fixed-point pixel sums -> float image times the sensor response
+// (render.h:1405-1409); accumulate != 0 adds to what dst holds
+__global__ void resolve_pixels(const long long* __restrict__ pix, float* __restrict__ dst, int n3, int accumulate,
+                               float sensor) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n3) return;
+  const float v = __ll2float_rn(pix[i]) * kPixelInvF * sensor;
+  dst[i] = accumulate ? dst[i] + v : v;
+}
+
+// scratch: the pixel sums and the sample counter (zeroed by the launch), then the pool
+static size_t pixel_bytes(const RenderCfg& cfg) { return (24 * (size_t)cfg.width * cfg.height + 16 + 255) / 256 * 256; }
+
+size_t plain_scratch_bytes(const RenderCfg& cfg) {
+  const BlockShape b = block_shape((unsigned long long)cfg.spp * cfg.width * cfg.height, sm_count());
+  return pixel_bytes(cfg) + block_pool_bytes((size_t)b.blocks * b.slots);
+}
+
+cudaError_t launch_plain(const DevScene& S, const RenderCfg& cfg, void* scratch, float* dst, int accumulate,
+                         uint32_t* err, unsigned long long* counters, cudaStream_t stream) {
+  const size_t n3 = 3 * (size_t)cfg.width * cfg.height;
+  PlainFrame F;
+  F.pix = static_cast<long long*>(scratch);
+  F.next = reinterpret_cast<unsigned long long*>(F.pix + n3);
+  F.samples = (unsigned long long)cfg.spp * cfg.width * cfg.height;
+  cudaError_t e = cudaMemsetAsync(scratch, 0, pixel_bytes(cfg), stream);
+  if (e != cudaSuccess) return e;
+  const BlockShape b = block_shape(F.samples, sm_count());
+  BlockPool P = block_pool(static_cast<char*>(scratch) + pixel_bytes(cfg), (size_t)b.blocks * b.slots);
+  P.slots = b.slots;
+  P.slots_used = b.used;
+  const size_t smem = block_shared_bytes(b.slots);
+  if (S.has_glossy || S.n_point_lights > 0 || S.has_tex)
+    pt_block<true><<<b.blocks, b.threads, smem, stream>>>(S, cfg, F, P, err, counters);
+  else
+    pt_block<false><<<b.blocks, b.threads, smem, stream>>>(S, cfg, F, P, err, counters);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  resolve_pixels<<<(unsigned int)((n3 + 255) / 256), 256, 0, stream>>>(F.pix, dst, (int)n3, accumulate, cfg.sensor);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_megakernel(const DevScene& S, const RenderCfg& cfg, float* out, uint32_t* err,

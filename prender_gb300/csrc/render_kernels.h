@@ -30,6 +30,12 @@ struct RenderCfg {
 cudaError_t launch_megakernel(const DevScene& S, const RenderCfg& cfg, float* out, uint32_t* err,
                               unsigned long long* counters, cudaStream_t stream);
 cudaError_t launch_reduce(const float* partial, float* dst, int n3, int chunks, int accumulate, cudaStream_t stream);
+// the plain form of scenes without subsurface materials: one kernel and the
+// resolve into dst; scratch (plain_scratch_bytes) holds the pixel sums
+// and the blocks' path slots
+size_t plain_scratch_bytes(const RenderCfg& cfg);
+cudaError_t launch_plain(const DevScene& S, const RenderCfg& cfg, void* scratch, float* dst, int accumulate,
+                          uint32_t* err, unsigned long long* counters, cudaStream_t stream);
 // 8-bit bitmap rows of a float image (output.cu)
 cudaError_t launch_to_rgb8(const float* rgb, int width, int height, double gamma_offset, uint8_t* out,
                            cudaStream_t stream);
