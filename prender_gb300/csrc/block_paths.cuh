@@ -280,21 +280,15 @@ inline BlockShape block_shape(unsigned long long samples, int sms) {
   BlockShape b;
   // small: every resident slot would take fewer than two samples
   b.threads = samples < 2ull * sms * kBlockThreads * kSlotsPerThread ? kSmallBlockThreads : kBlockThreads;
-  b.slots = kSlotsPerThread * b.threads;
+  const unsigned long long room = kSlotsPerThread * b.threads;
   const unsigned long long most = (unsigned long long)sms * (kBlockThreads / b.threads);
   unsigned long long used = (samples + most - 1) / most;
-  used = used < 16 ? 16 : used > (unsigned long long)b.slots ? b.slots : used;
+  used = used < 16 ? 16 : used > room ? room : used;
   const unsigned long long want = (samples + used - 1) / used;
   b.blocks = (unsigned int)(want < most ? want : most);
   b.used = (int)used;
+  b.slots = (b.used + 15) / 16 * 16;
   return b;
-}
-inline int sm_count() {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    sms = 152;
-  return sms;
 }
 
 // bytes of a pool of n slots, and its arrays in a buffer of that size

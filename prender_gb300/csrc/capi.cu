@@ -298,6 +298,9 @@ static int build_device_scene(pr_ctx* c, const pr_scene_desc* d, SceneObjData& o
   o.kerr = h.kerr;
   o.kerr.texture = h.kerr_texture.empty() ? nullptr : (const unsigned char*)o.kerr_tex.p;
   o.kerr.disk_tex = h.kerr_disk_texture.empty() ? nullptr : (const uchar4*)o.kerr_disk_tex.p;
+  o.kerr.rms_f = (float)o.kerr.Rmstable;
+  o.kerr.a2_f = (float)o.kerr.a2;
+  for (int k = 0; k < 3; k++) o.kerr.pos_f[k] = (float)o.kerr.pos[k];
   DevScene& S = o.dev;
   memset(&S, 0, sizeof(S));
   S.ents = (const GEntity*)o.ents.p;
@@ -361,6 +364,13 @@ static int build_device_scene(pr_ctx* c, const pr_scene_desc* d, SceneObjData& o
     f.face_base = e.face_base;
     f.node_base = e.rnode_base;
     f.sss_rmax = (float)e.sss_rmax;
+    if (e.type == PR_ENT_CIRCLE) {
+      for (int k = 0; k < 3; k++) {
+        f.u[k] = e.du_len > 0.0 ? (float)(e.du_axis[k] / e.du_len) : 0.0f;
+        f.v[k] = e.dv_len > 0.0 ? (float)(e.dv_axis[k] / e.dv_len) : 0.0f;
+      }
+      f.node_base = e.kerr_disk;
+    }
   }
   sphere_bounds(h, S);
   mesh_bounds(h, S);
@@ -911,14 +921,15 @@ int pr_render_dev(pr_ctx* c, const pr_camera* cam, const pr_render_params* p, fl
   uint64_t mlt_paths = 0, mlt_launches = 0;
   if (kerr || worm) {
     // every scene query of a Kerr or wormhole scene is a geodesic trace: one form only
-    PR_CUDA(c, c->partial.ensure(sizeof(float) * n3 * (size_t)g.chunks));
-    if (kerr)
-      PR_CUDA(c, launch_kerr_render(c->cur.dev, c->cur.kerr, g, (float*)c->partial.p, (uint32_t*)c->errword.p,
-                                    (unsigned long long*)c->counters.p, c->stream));
-    else
-      PR_CUDA(c, launch_worm_render(c->cur.dev, c->cur.worm, g, (float*)c->partial.p, (uint32_t*)c->errword.p,
-                                    (unsigned long long*)c->counters.p, c->stream));
-    PR_CUDA(c, launch_reduce((const float*)c->partial.p, rgb_dev, (int)n3, g.chunks, accumulate, c->stream));
+    if (kerr) {
+      PR_CUDA(c, c->partial.ensure(kerr_scratch_bytes(c->cur.kerr, g)));
+      PR_CUDA(c, launch_kerr_render(c->cur.dev, c->cur.kerr, g, c->partial.p, rgb_dev, accumulate,
+                                    (uint32_t*)c->errword.p, (unsigned long long*)c->counters.p, c->stream));
+    } else {
+      PR_CUDA(c, c->partial.ensure(worm_scratch_bytes(g)));
+      PR_CUDA(c, launch_worm_render(c->cur.dev, c->cur.worm, g, c->partial.p, rgb_dev, accumulate,
+                                    (uint32_t*)c->errword.p, (unsigned long long*)c->counters.p, c->stream));
+    }
   } else if (p->mode == PR_MODE_MLT) {
     st = render_mlt(c, g, p, rgb_dev, accumulate, mlt_paths, mlt_launches);
     if (st != PR_OK) return st;
@@ -947,7 +958,7 @@ int pr_render_dev(pr_ctx* c, const pr_camera* cam, const pr_render_params* p, fl
   const uint64_t paths = wf ? (uint64_t)g.spp * g.width * g.height : mlt ? mlt_paths : cnt[0];
   // wavefront: reset per pass + 4 per iteration + resolve; megakernel: kernel + reduce;
   // MLT: bootstrap, chain start, the chains' launches, resolve
-  const uint64_t launches = wf ? 4 * cnt[5] + c->wf_passes + 1 : mlt ? mlt_launches : 2;
+  const uint64_t launches = wf ? 4 * cnt[5] + c->wf_passes + 1 : mlt ? mlt_launches : kerr ? (uint64_t)kerr_render_launches(c->cur.kerr) : 2;
   // Kerr counters: [1] accepted RK steps, [2] RK attempts, [3] segment scene
   // tests, reported as pr_kerr_trace does (segments, nodes_visited, tri_tests)
   c->stats = kerr ? pr_render_stats{paths, cnt[3], cnt[1], cnt[2], ms, launches}
@@ -1425,7 +1436,9 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
   PR_CUDA(c, cudaSetDevice(c->device));
   cudaGetLastError();  // an error left by an unrelated earlier call is not this call's
   std::vector<RenderCfg> cfg((size_t)n);
-  std::vector<size_t> off((size_t)n + 1, 0);
+  // the jobs of a branch run one after another and share its scratch
+  const int n_streams = std::min(n, 16);
+  std::vector<size_t> branch_room((size_t)n_streams, 0), off((size_t)n_streams + 1, 0);
   uint64_t paths = 0;
   bool all_kerr = true;
   for (int j = 0; j < n; j++) {
@@ -1443,8 +1456,11 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
     const SceneObjData& sc = J.scene->data;
     size_t bytes = sizeof(float) * (size_t)cfg[j].width * cfg[j].height * 3 * (size_t)cfg[j].chunks;
     if (J.params.mode == PR_MODE_WAVEFRONT && !sc.kerr.enabled && !sc.worm.enabled) bytes = 0;
+    else if (sc.kerr.enabled) bytes = kerr_scratch_bytes(sc.kerr, cfg[j]);
+    else if (sc.worm.enabled) bytes = worm_scratch_bytes(cfg[j]);
     else if (streamed(sc)) bytes = plain_scratch_bytes(cfg[j]);
-    off[j + 1] = off[j] + (bytes + 255) / 256 * 256;
+    size_t& room = branch_room[j % n_streams];
+    room = std::max(room, (bytes + 255) / 256 * 256);
     paths += (uint64_t)cfg[j].spp * cfg[j].width * cfg[j].height;
   }
   // jobs in the wavefront form share the context's path pool: they run one
@@ -1453,8 +1469,8 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
   for (int j = 0; j < n; j++)
     wf_job[j] = jobs[j].params.mode == PR_MODE_WAVEFRONT && !jobs[j].scene->data.kerr.enabled &&
                 !jobs[j].scene->data.worm.enabled;
-  PR_CUDA(c, c->batch_partial.ensure(std::max<size_t>(off[n], 1)));
-  const int n_streams = std::min(n, 16);
+  for (int k = 0; k < n_streams; k++) off[k + 1] = off[k] + branch_room[k];
+  PR_CUDA(c, c->batch_partial.ensure(std::max<size_t>(off[n_streams], 1)));
   while ((int)c->batch_streams.size() < n_streams) {
     cudaStream_t st;
     PR_CUDA(c, cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
@@ -1480,20 +1496,23 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
     cudaStream_t st = c->batch_streams[j % n_streams];
     const SceneObjData& sc = J.scene->data;
     const int n3 = cfg[j].width * cfg[j].height * 3;
-    float* partial = (float*)(part + off[j]);
+    float* partial = (float*)(part + off[j % n_streams]);
     if (streamed(sc)) {
       e = launch_plain(sc.dev, cfg[j], partial, J.rgb_dev, J.accumulate, (uint32_t*)c->errword.p,
                         (unsigned long long*)c->counters.p, st);
       continue;
     }
-    if (sc.kerr.enabled)
-      e = launch_kerr_render(sc.dev, sc.kerr, cfg[j], partial, (uint32_t*)c->errword.p,
+    if (sc.kerr.enabled) {
+      e = launch_kerr_render(sc.dev, sc.kerr, cfg[j], partial, J.rgb_dev, J.accumulate, (uint32_t*)c->errword.p,
                              (unsigned long long*)c->counters.p, st);
-    else if (sc.worm.enabled)
-      e = launch_worm_render(sc.dev, sc.worm, cfg[j], partial, (uint32_t*)c->errword.p,
+      continue;
+    }
+    if (sc.worm.enabled) {
+      e = launch_worm_render(sc.dev, sc.worm, cfg[j], partial, J.rgb_dev, J.accumulate, (uint32_t*)c->errword.p,
                              (unsigned long long*)c->counters.p, st);
-    else
-      e = launch_megakernel(sc.dev, cfg[j], partial, (uint32_t*)c->errword.p,
+      continue;
+    }
+    e = launch_megakernel(sc.dev, cfg[j], partial, (uint32_t*)c->errword.p,
                             (unsigned long long*)c->counters.p, st);
     if (e == cudaSuccess) e = launch_reduce(partial, J.rgb_dev, n3, cfg[j].chunks, J.accumulate, st);
   }
@@ -1530,7 +1549,7 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
   uint64_t launches = 0, wf_passes = 0;
   for (int j = 0; j < n; j++) {
     if (!wf_job[j]) {
-      launches += 2;
+      launches += jobs[j].scene->data.kerr.enabled ? (uint64_t)kerr_render_launches(jobs[j].scene->data.kerr) : 2;
       continue;
     }
     const int stw = render_wavefront(c, cfg[j], jobs[j].rgb_dev, jobs[j].accumulate, &jobs[j].scene->data);

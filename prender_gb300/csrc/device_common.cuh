@@ -334,13 +334,13 @@ __device__ inline bool exact_qbvh(const DevScene& S, const GEntity& e, const Exa
 // The default hit-shading hook of exact_closest: no entity rewrites its hit.
 struct NoHitShading {
   __device__ __forceinline__ void begin() {}
-  __device__ __forceinline__ bool circle(const GEntity&, dv3) { return true; }
+  __device__ __forceinline__ bool circle(const GEntity&, dv3, double) { return true; }
   __device__ __forceinline__ void best(const GEntity&) {}
 };
 
 // intersect_scene_ (scene.cpp:83-173): push the origin 1e-6 along the
 // direction, loop over entities, keep the strictly closest.  hs sees every
-// disk hit (at its hit point) before it competes for the closest, as
+// disk hit (its hit point and distance) before it competes for the closest, as
 // Circle::intersect's own texture branch does (circle.h:177-335), and is told
 // which entity ends up closest.
 template <class HS>
@@ -364,7 +364,7 @@ __device__ inline bool exact_closest_hs(const DevScene& S, dv3 org, dv3 dir, dou
     } else if (e.type == PR_ENT_CIRCLE) {
       got = exact_circle(e, o2, dir, t);
       // the hit point exactly as exact_circle forms it
-      if (got) got = hs.circle(e, {da(dm(dir.x, t), o2.x), da(dm(dir.y, t), o2.y), da(dm(dir.z, t), o2.z)});
+      if (got) got = hs.circle(e, {da(dm(dir.x, t), o2.x), da(dm(dir.y, t), o2.y), da(dm(dir.z, t), o2.z)}, t);
     } else if (e.type == PR_ENT_POLYGON) {
       if (!ray_ready) {
         r = make_exact_ray(o2, dir);

@@ -20,18 +20,22 @@ struct KerrOut {
   double* hit_t;
 };
 
-// counters[0] rays, [1] accepted steps, [2] RK45 attempts, [3] segment tests
+// counters[0] rays, [1] accepted steps, [2] RK45 attempts, [3] segment tests,
+// [kKerrNextCounter] (zero before) the rays handed out
+constexpr int kKerrNextCounter = 15;
 cudaError_t launch_kerr_trace_fp64(const DevScene& S, const GKerr& K, const double* rays, int64_t n, KerrOut out,
                                    uint32_t* err, unsigned long long* counters, cudaStream_t stream);
 cudaError_t launch_kerr_trace_fp32(const DevScene& S, const GKerr& K, const double* rays, int64_t n, KerrOut out,
                                    uint32_t* err, unsigned long long* counters, cudaStream_t stream);
 
-// the renderer with every scene query traced along a geodesic; same output
-// layout as launch_megakernel (per-chunk partial images)
-cudaError_t launch_kerr_render_fp64(const DevScene& S, const GKerr& K, const RenderCfg& cfg, float* partial,
-                                    uint32_t* err, unsigned long long* counters, cudaStream_t stream);
-cudaError_t launch_kerr_render_fp32(const DevScene& S, const GKerr& K, const RenderCfg& cfg, float* partial,
-                                    uint32_t* err, unsigned long long* counters, cudaStream_t stream);
+// the renderer with every scene query traced along a geodesic, into dst
+// (scratch of kerr_scratch_bytes); kerr_render_launches kernels
+size_t kerr_scratch_bytes_fp64(const RenderCfg& cfg);
+size_t kerr_scratch_bytes_fp32(const RenderCfg& cfg);
+cudaError_t launch_kerr_render_fp64(const DevScene& S, const GKerr& K, const RenderCfg& cfg, void* scratch, float* dst,
+                                    int accumulate, uint32_t* err, unsigned long long* counters, cudaStream_t stream);
+cudaError_t launch_kerr_render_fp32(const DevScene& S, const GKerr& K, const RenderCfg& cfg, void* scratch, float* dst,
+                                    int accumulate, uint32_t* err, unsigned long long* counters, cudaStream_t stream);
 
 // forward-mode ray-bundle Jacobian (kerr_sens.cu); any output may be null
 cudaError_t launch_kerr_sensitivity(const DevScene& S, const GKerr& K, const double* rays, const double* basis,
@@ -47,10 +51,17 @@ inline cudaError_t launch_kerr_trace(const DevScene& S, const GKerr& K, const do
   return K.precision == PR_KERR_FP32 ? launch_kerr_trace_fp32(S, K, rays, n, out, err, counters, stream)
                                      : launch_kerr_trace_fp64(S, K, rays, n, out, err, counters, stream);
 }
-inline cudaError_t launch_kerr_render(const DevScene& S, const GKerr& K, const RenderCfg& cfg, float* partial,
-                                      uint32_t* err, unsigned long long* counters, cudaStream_t stream) {
-  return K.precision == PR_KERR_FP32 ? launch_kerr_render_fp32(S, K, cfg, partial, err, counters, stream)
-                                     : launch_kerr_render_fp64(S, K, cfg, partial, err, counters, stream);
+inline size_t kerr_scratch_bytes(const GKerr& K, const RenderCfg& cfg) {
+  return K.precision == PR_KERR_FP32 ? kerr_scratch_bytes_fp32(cfg) : kerr_scratch_bytes_fp64(cfg);
+}
+// kernel and resolve; the mixed form's far field is a kernel of its own
+inline int kerr_render_launches(const GKerr& K) { return K.precision == PR_KERR_FP32 ? 3 : 2; }
+inline cudaError_t launch_kerr_render(const DevScene& S, const GKerr& K, const RenderCfg& cfg, void* scratch, float* dst,
+                                      int accumulate, uint32_t* err, unsigned long long* counters,
+                                      cudaStream_t stream) {
+  return K.precision == PR_KERR_FP32
+             ? launch_kerr_render_fp32(S, K, cfg, scratch, dst, accumulate, err, counters, stream)
+             : launch_kerr_render_fp64(S, K, cfg, scratch, dst, accumulate, err, counters, stream);
 }
 
 }  // namespace pr

@@ -12,17 +12,26 @@ namespace pr {
 cudaError_t launch_kerr_trace_fp32(const DevScene& S, const GKerr& K, const double* rays, int64_t n, KerrOut out,
                                    uint32_t* err, unsigned long long* counters, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
-  const int64_t blocks = (n + 127) / 128;
-  kerr_trace_kernel<true><<<(unsigned)blocks, 128, 0, stream>>>(S, K, rays, n, out, err, counters);
+  kerr_trace_kernel<true><<<geodesic_blocks((unsigned long long)n, sm_count()), 128, 0, stream>>>(S, K, rays, n, out,
+                                                                                              err, counters);
   return cudaGetLastError();
 }
 
-cudaError_t launch_kerr_render_fp32(const DevScene& S, const GKerr& K, const RenderCfg& cfg, float* partial,
-                                    uint32_t* err, unsigned long long* counters, cudaStream_t stream) {
-  const uint64_t threads = (uint64_t)cfg.tiles_x * cfg.tiles_y * 32ull * (uint64_t)cfg.chunks;
-  const uint32_t blocks = (uint32_t)((threads + 127) / 128);
-  kerr_render_kernel<true><<<blocks, 128, 0, stream>>>(S, K, cfg, partial, err, counters);
-  return cudaGetLastError();
+size_t kerr_scratch_bytes_fp32(const RenderCfg& cfg) { return kerr_zero_bytes(cfg) + sizeof(KerrFar) * kerr_far_cap(cfg); }
+
+cudaError_t launch_kerr_render_fp32(const DevScene& S, const GKerr& K, const RenderCfg& cfg, void* scratch, float* dst,
+                                    int accumulate, uint32_t* err, unsigned long long* counters, cudaStream_t stream) {
+  cudaError_t e = cudaMemsetAsync(scratch, 0, kerr_zero_bytes(cfg), stream);
+  if (e != cudaSuccess) return e;
+  const KerrFrame F = kerr_frame(cfg, scratch, true);
+  const int sms = sm_count();
+  kerr_render_kernel<1><<<geodesic_blocks(F.samples, sms), 128, 0, stream>>>(S, K, cfg, F, err, counters);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  kerr_render_kernel<2><<<geodesic_blocks(F.far_cap, sms), 128, 0, stream>>>(S, K, cfg, F, err, counters);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  return launch_resolve(F.pix, dst, 3 * cfg.width * cfg.height, accumulate, cfg.sensor, stream);
 }
 
 }  // namespace pr

@@ -12,6 +12,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "geodesic_math.cuh"
 #include "kerr.h"
 #include "path_logic.cuh"
 
@@ -42,11 +43,19 @@ __device__ __forceinline__ void cart_to_bl(double x, double y, double z, double 
   ph = phi;
 }
 
-// Spherical::ToBoyerLindquist (vector3d.h:888-898): BL (r, theta, phi) -> Cartesian
-__device__ __forceinline__ dv3 bl_to_cart(double r, double th, double ph, double a) {
+// Spherical::ToBoyerLindquist (vector3d.h:888-898): BL (r, theta, phi) ->
+// Cartesian.  (sincos gives the bits of sin and of cos for two thirds of the
+// FP64 instructions of both.)
+__device__ __forceinline__ dv3 bl_to_cart(double r, double sint, double cost, double ph, double a) {
   const double rr = sqrt(r * r + a * a);
-  const double sint = sin(th);
-  return {rr * cos(ph) * sint, rr * sin(ph) * sint, r * cos(th)};
+  double sinp, cosp;
+  sincos(ph, &sinp, &cosp);
+  return {rr * cosp * sint, rr * sinp * sint, r * cost};
+}
+__device__ __forceinline__ dv3 bl_to_cart(double r, double th, double ph, double a) {
+  double sint, cost;
+  sincos(th, &sint, &cost);
+  return bl_to_cart(r, sint, cost, ph, a);
 }
 
 // Cartesian::ToSpherical (vector3d.h:900-918), angles only
@@ -81,17 +90,19 @@ struct KerrRay {
   double a, a2, M;
   double L, kappa;
 
-  // geodesic (KerrBlackHole.h:1239-1281)
+  // geodesic (KerrBlackHole.h:1239-1281); the second form is given sin and cos of theta
   __device__ __forceinline__ void geodesic(const double* y, double* dydx) const {
+    double sintheta, costheta;
+    sincos(y[1], &sintheta, &costheta);
+    geodesic(y, sintheta, costheta, dydx);
+  }
+  __device__ __forceinline__ void geodesic(const double* y, double sintheta, double costheta, double* dydx) const {
     const double r = y[0];
-    const double theta = y[1];
     const double pr = y[4];
     const double ptheta = y[5];
     const double r2 = r * r;
     const double twor = 2.0 * M * r;
-    const double sintheta = sin(theta);
     double sin2 = sintheta * sintheta;
-    const double costheta = cos(theta);
     const double cos2 = costheta * costheta;
     const double sigma = r2 + a2 * cos2;
     const double delta = r2 - twor + a2;
@@ -172,8 +183,9 @@ struct KerrRay {
   }
 
   // NextPosition + rkqs (KerrBlackHole.h:471-522, :1366-1431): one accepted
-  // step from y (escal 1e11, at most 40 shrinking retries); returns hnext
-  __device__ __forceinline__ double next_position(double* y, const double* dydx, double htry,
+  // step from y (escal 1e11, at most 40 shrinking retries); returns the next
+  // step, at most cap
+  __device__ __forceinline__ double next_position(double* y, const double* dydx, double htry, double cap,
                                                   uint32_t& attempts, double* errmax_out = nullptr) const {
     double yscal[6];
 #pragma unroll
@@ -184,12 +196,7 @@ struct KerrRay {
     for (int loop = 0; loop < 40; loop++) {
       rkstep(y, dydx, h, ytemp, yerr);
       attempts++;
-      errmax = 0.0;
-#pragma unroll
-      for (int i = 0; i < 6; i++) {
-        const double temp = fabs(yerr[i] / yscal[i]);
-        if (temp > errmax) errmax = temp;
-      }
+      errmax = max_ratio<6>(yerr, yscal);
       errmax *= escal;
       if (errmax <= 1.0) break;
       const double htemp = 0.9 * h / sqrt(sqrt(errmax));
@@ -200,9 +207,7 @@ struct KerrRay {
         if (htemp < h) h = htemp;
       }
     }
-    double hnext;
-    if (errmax > 1.89e-4) hnext = 0.9 * h * pow(errmax, -0.2);
-    else hnext = 5.0 * h;
+    const double hnext = next_step(h, errmax, cap);
     if (errmax_out) *errmax_out = errmax;
 #pragma unroll
     for (int i = 0; i < 6; i++) y[i] = ytemp[i];
@@ -294,7 +299,6 @@ struct KerrHit {
   double t;        // hit distance along the last segment
   dv3 seg_o;       // origin of the segment the hit lies on (before the 1e-6 push)
   dv3 dir2;        // last polyline direction
-  double y[6];     // final state
   bool ov;         // status 1 on the accretion disk: its rewritten colour / emission
   float3 ovc, ove;
 };
@@ -359,7 +363,9 @@ __device__ inline void disk_doppler(double c[3], double d, double effect) {
 // The deterministic part of the disk branch at world point p: false where
 // the disk is not there (inside the horizon or the ISCO, beyond its radius,
 // off the texture); else colour, emission and alpha (circle.h:244-322).
-__device__ inline bool kerr_disk_shade(const GKerr& K, const GEntity& e, dv3 p, double col[3], double em[3],
+// In two parts: the texel with its temperature and alpha, which decide whether
+// the hit counts, and the Doppler shift (most of the work) of a hit that does.
+__device__ inline bool kerr_disk_texel(const GKerr& K, const GEntity& e, dv3 p, double col[3], double em[3],
                                        double& alp) {
   const double rx = p.x - K.pos[0], ry = p.y - K.pos[1], rz = p.z - K.pos[2];
   double sr, sth, sph;
@@ -409,6 +415,12 @@ __device__ inline bool kerr_disk_shade(const GKerr& K, const GEntity& e, dv3 p, 
   alp = t.w / 255.0;
   const double cl = sqrt((col[0] * col[0] + col[2] * col[2]) + col[1] * col[1]) / 3.0;
   if (cl < alp) alp = cl;  // std::min(alpha, |colour| / 3)
+  return true;
+}
+
+__device__ inline void kerr_disk_shift(const GKerr& K, dv3 p, double col[3], double em[3]) {
+  const double rx = p.x - K.pos[0], ry = p.y - K.pos[1], rz = p.z - K.pos[2];
+  const double tmp_r = sqrt((rx * rx + rz * rz) + ry * ry);
   // the disk's orbital velocity (getDiskVelocity about +z with sign -1,
   // KerrBlackHole.h:1507-1531) scaled to the circular-orbit speed seen by a
   // locally non-rotating observer (circle.h:292-302)
@@ -462,8 +474,16 @@ __device__ inline bool kerr_disk_shade(const GKerr& K, const GEntity& e, dv3 p, 
   }
   disk_doppler(col, dop, K.doppler_effect);
   disk_doppler(em, dop, K.doppler_effect);
+}
+
+__device__ inline bool kerr_disk_shade(const GKerr& K, const GEntity& e, dv3 p, double col[3], double em[3],
+                                       double& alp) {
+  if (!kerr_disk_texel(K, e, p, col, em, alp)) return false;
+  kerr_disk_shift(K, p, col, em);
   return true;
 }
+
+constexpr double kSegment = 2.0;  // h_dist: the longest step, and how far a segment test looks
 
 // exact_closest hook of the Kerr tracer: a disk_map disk is there only where
 // its texture is and its alpha test passes; the closest hit on it carries the
@@ -475,13 +495,14 @@ struct KerrDiskShading {
   bool cand, ov;
   float3 cc, ce, oc, oe;
   __device__ __forceinline__ void begin() { ov = false; }
-  __device__ __forceinline__ bool circle(const GEntity& e, dv3 p) {
+  __device__ __forceinline__ bool circle(const GEntity& e, dv3 p, double t) {
     cand = false;
     if (!e.kerr_disk || !K->disk_tex) return true;
     double col[3], em[3], alp;
-    if (!kerr_disk_shade(*K, e, p, col, em, alp)) return false;
+    if (!kerr_disk_texel(*K, e, p, col, em, alp)) return false;
     if (alp == 0.0) return false;
     if (alp < 0.99 && alp <= (double)rng->next()) return false;
+    if (t < kSegment) kerr_disk_shift(*K, p, col, em);  // a hit beyond the segment is not kept
     cand = true;
     cc = f3((float)col[0], (float)col[1], (float)col[2]);
     ce = f3((float)em[0], (float)em[1], (float)em[2]);
@@ -494,151 +515,15 @@ struct KerrDiskShading {
   }
 };
 
+__device__ __forceinline__ DiskAlpha disk_alpha(const GKerr& K) {
+  return DiskAlpha{K.disk_tex, K.disk_w, K.disk_h, K.use_temp == 0, K.rms_f, K.a2_f, {K.pos_f[0], K.pos_f[1], K.pos_f[2]}};
+}
+
 // the key of the alpha-test stream: the render seed mixed with the disk seed
 __device__ __forceinline__ uint64_t disk_stream_key(uint64_t seed, const GKerr& K) {
   return seed ^ (K.disk_seed * 0x9E3779B97F4A7C15ull);
 }
 constexpr uint32_t kDiskBranch = 0xFFFFFFFFu;  // counter lane of the alpha-test stream
-
-// the Kerr branch of intersect_scene for one ray (scene.cpp:448-732)
-template <class HS>
-__device__ void kerr_trace_ray(const DevScene& S, const GKerr& K, dv3 org, dv3 dir, KerrHit& out, KerrCount& cnt,
-                               uint32_t* err, HS& hs) {
-  KerrRay k{K.a, K.a2, K.M, 0.0, 0.0};
-  double* y = out.y;
-  double dydx[6];
-  const dv3 rel = {org.x - K.pos[0], org.y - K.pos[1], org.z - K.pos[2]};  // Setup (KerrBlackHole.h:153-166)
-  double r0, th0, ph0;
-  cart_to_bl(rel.x, rel.y, rel.z, K.a, r0, th0, ph0);
-  y[0] = r0;
-  y[1] = th0;
-  y[2] = ph0;
-  y[3] = 0;
-  y[4] = 0;
-  y[5] = 0;
-  out.steps = 0;
-  out.ov = false;
-  out.ent = -1;
-  out.prim = -1;
-  out.t = -1.0;
-  out.dir2 = dir;
-  out.seg_o = org;
-  if (r0 < K.Rhor) {
-    out.status = 2;
-    return;
-  }
-  k.initial(dir, y, dydx, r0, th0);
-  const double h_dist = 2.0;
-  double h_step = h_dist;
-  dv3 org1 = org, org2 = org, dir2 = dir;
-  int c = 0;
-  while (c < K.max_steps) {
-    double t;
-    int ent, prim;
-    cnt.segments++;
-    if (exact_closest_hs(S, org1, dir2, t, ent, prim, err, cnt.nodes, cnt.tris, hs)) {
-      if (t < h_dist) {
-        // hit point of intersect_scene_: (org1 + 1e-6 dir2) + t dir2
-        const dv3 o2 = dadd3(org1, dscale3(dir2, 0.000001));
-        const dv3 p = {o2.x + t * dir2.x, o2.y + t * dir2.y, o2.z + t * dir2.z};
-        double sr, sth, sph;
-        cart_to_bl(p.x - K.pos[0], p.y - K.pos[1], p.z - K.pos[2], K.a, sr, sth, sph);
-        out.steps = c;
-        out.dir2 = dir2;
-        out.seg_o = org1;
-        if (sr < K.Rhor) {
-          out.status = 2;
-        } else {
-          out.status = 1;
-          out.ent = ent;
-          out.prim = prim;
-          out.t = t;
-          out.ov = hs.ov;
-          out.ovc = hs.oc;
-          out.ove = hs.oe;
-        }
-        return;
-      }
-    }
-    k.geodesic(y, dydx);
-    if (fabs(h_step) < 1.0e-10) {
-      out.status = 4;
-      out.steps = c;
-      out.dir2 = dir2;
-      return;
-    }
-    const double r_before = y[0];
-    h_step = k.next_position(y, dydx, h_step, cnt.attempts);
-    if (h_step > h_dist) h_step = h_dist;
-    if (y[0] < K.Rhor) {
-      out.status = 2;
-      out.steps = c;
-      out.dir2 = dir2;
-      return;
-    }
-    org1 = org2;
-    const dv3 q = bl_to_cart(y[0], y[1], y[2], K.a);
-    org2 = {q.x + K.pos[0], q.y + K.pos[1], q.z + K.pos[2]};
-    dir2 = dnormalize({org2.x - org1.x, org2.y - org1.y, org2.z - org1.z});
-    c++;
-    cnt.steps++;
-    // optional early exit (not in the reference): far out and receding
-    if (K.escape_radius > 0.0 && y[0] > K.escape_radius && y[0] > r_before) break;
-  }
-  out.steps = c;
-  out.dir2 = dir2;
-  out.seg_o = org2;
-  double t;
-  int ent, prim;
-  cnt.segments++;
-  if (exact_closest_hs(S, org2, dir2, t, ent, prim, err, cnt.nodes, cnt.tris, hs)) {
-    out.status = 5;
-    out.ent = ent;
-    out.prim = prim;
-    out.t = t;
-  } else {
-    out.status = 0;
-  }
-}
-
-// background map lookup of an escaped ray (scene.cpp:711-727; SphericalMapping::Map, circle.h:92-105)
-__device__ __forceinline__ float3 kerr_background(const GKerr& K, const double* yy, const float* bg) {
-  if (!K.texture) return f3(bg[0], bg[1], bg[2]);
-  double y1 = yy[1] * K.map_coef[0] + K.map_coef[1];
-  double y2 = yy[2] * K.map_coef[2] + K.map_coef[3];
-  y1 = fmod(y1, kPi);
-  y2 = fmod(y2, 2.0 * kPi);
-  double phi = y2, theta = y1;
-  if (phi < 0.0) phi += 2.0 * kPi;
-  if (theta < 0.0) theta = -theta;
-  int x = (int)(phi / (2.0 * kPi) * K.tex_w);
-  x = ((x % K.tex_w) + K.tex_w) % K.tex_w;  // in range for any input, NaN included
-  int yv = (int)(theta / kPi * K.tex_h);
-  yv = ((yv % K.tex_h) + K.tex_h) % K.tex_h;
-  const unsigned char* t = K.texture + 3 * ((size_t)yv * K.tex_w + x);
-  return f3((float)(K.texture_coef * t[0] / 255.0), (float)(K.texture_coef * t[1] / 255.0),
-            (float)(K.texture_coef * t[2] / 255.0));
-}
-
-template <class T>
-__device__ __forceinline__ T warp_sum(T v) {
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-  return v;
-}
-
-__device__ __forceinline__ void flush_counts(const KerrCount& c, uint32_t rays, unsigned long long* counters) {
-  if (!counters) return;
-  const unsigned long long a = warp_sum<unsigned long long>(rays), b = warp_sum<unsigned long long>(c.steps),
-                           d = warp_sum<unsigned long long>(c.attempts),
-                           e = warp_sum<unsigned long long>(c.segments);
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(counters + 0, a);
-    atomicAdd(counters + 1, b);
-    atomicAdd(counters + 2, d);
-    atomicAdd(counters + 3, e);
-  }
-}
-
 
 // ======================================================================
 // Mixed-precision form (pr_kerr.precision = PR_KERR_FP32).  GB300 runs FP32
@@ -744,9 +629,26 @@ __device__ __forceinline__ double radial_potential(double r, double a, double L,
   return w * w - delta * (kappa - 2.0 * a * L);
 }
 
-// no turning point between the horizon and r: R > 0 on a fine grid of [r+, r]
+// no turning point between the horizon and r: R > 0 on a fine grid of [r+, r].
+// FP32 decides where R's sign clears its rounding (all but rays within about
+// 1e-5 of critical), FP64 the rest.
 __device__ __forceinline__ bool no_turning_point(double r, double rplus, double a, double L, double kappa) {
   const int n = 64;
+  {
+    const float rp = (float)rplus, dr = (float)(r - rplus), af = (float)a, aL = (float)(a * L);
+    const float q = (float)(kappa - 2.0 * a * L), a2 = af * af;
+    bool clear = true;
+    for (int i = 0; i <= n; i++) {
+      const float rr = rp + dr * ((float)i / n), r2 = rr * rr;
+      const float w = r2 + a2 - aL, delta = r2 - 2.0f * rr + a2;
+      const float R = w * w - delta * q;
+      // the sums' terms, and R's change over the rounding of rr
+      const float m = r2 + a2 + fabsf(aL), e = 1.0e-5f * (m * m + (r2 + 2.0f * rr + a2) * fabsf(q));
+      if (R < -e) return false;
+      clear = clear && R > e;
+    }
+    if (clear) return true;
+  }
   for (int i = 0; i <= n; i++) {
     const double rr = rplus + (r - rplus) * (double)i / n;
     if (!(radial_potential(rr, a, L, kappa) > 0.0)) return false;
@@ -754,22 +656,32 @@ __device__ __forceinline__ bool no_turning_point(double r, double rplus, double 
   return true;
 }
 
-// the Kerr branch of intersect_scene, mixed precision (see above)
-template <class HS>
-__device__ void kerr_trace_ray_fast(const DevScene& S, const GKerr& K, dv3 org, dv3 dir, KerrHit& out, KerrCount& cnt,
-                                    uint32_t* err, HS& hs, bool capture_shortcut) {
-  KerrRay k{K.a, K.a2, K.M, 0.0, 0.0};
-  double* y = out.y;
-  double dydx[6];
-  const dv3 rel = {org.x - K.pos[0], org.y - K.pos[1], org.z - K.pos[2]};
+// ---- the march of one ray ---------------------------------------------------
+// The state between the steps of the reference's loop (scene.cpp:448-732)
+struct KerrMarch {
+  KerrRay k;
+  double y[6];
+  double sint, cost;     // of y[1] (not kept up in the far field)
+  double h_step, errmax;
+  dv3 org1, org2, dir2;  // the polyline's last vertices and direction
+  double yprev[3];       // mixed form: the state before the last step
+  int c;                 // accepted steps
+  bool far_mode;         // mixed form: in the far field
+  bool capture_checked;
+};
+
+// Set-up of a ray; false if it starts inside the horizon (out says so)
+__device__ __forceinline__ bool kerr_start(const GKerr& K, dv3 org, dv3 dir, KerrMarch& M, KerrHit& out) {
+  M.k = KerrRay{K.a, K.a2, K.M, 0.0, 0.0};
+  const dv3 rel = {org.x - K.pos[0], org.y - K.pos[1], org.z - K.pos[2]};  // Setup (KerrBlackHole.h:153-166)
   double r0, th0, ph0;
   cart_to_bl(rel.x, rel.y, rel.z, K.a, r0, th0, ph0);
-  y[0] = r0;
-  y[1] = th0;
-  y[2] = ph0;
-  y[3] = 0;
-  y[4] = 0;
-  y[5] = 0;
+  M.y[0] = r0;
+  M.y[1] = th0;
+  M.y[2] = ph0;
+  M.y[3] = 0;
+  M.y[4] = 0;
+  M.y[5] = 0;
   out.steps = 0;
   out.ov = false;
   out.ent = -1;
@@ -779,122 +691,40 @@ __device__ void kerr_trace_ray_fast(const DevScene& S, const GKerr& K, dv3 org, 
   out.seg_o = org;
   if (r0 < K.Rhor) {
     out.status = 2;
-    return;
+    return false;
   }
-  k.initial(dir, y, dydx, r0, th0);
-  const KerrRayF kf{(float)K.a, (float)K.a2, (float)K.M, (float)k.L, (float)k.kappa};
-  const double far = fmax(kFarRadius, K.scene_radius + 2.0);
-  const double rplus = K.M + sqrt(K.M * K.M - K.a2);
-  bool capture_checked = false;
-  const double h_dist = 2.0;
-  double h_step = h_dist;
-  double errmax = 1.0;
-  dv3 org1 = org, org2 = org, dir2 = dir;
-  double yprev[3] = {y[0], y[1], y[2]};
-  bool far_mode = false;
-  int c = 0;
-  while (c < K.max_steps) {
-    if (!far_mode) {
-      double t;
-      int ent, prim;
-      cnt.segments++;
-      if (exact_closest_hs(S, org1, dir2, t, ent, prim, err, cnt.nodes, cnt.tris, hs)) {
-        if (t < h_dist) {
-          const dv3 o2 = dadd3(org1, dscale3(dir2, 0.000001));
-          const dv3 p = {o2.x + t * dir2.x, o2.y + t * dir2.y, o2.z + t * dir2.z};
-          double sr, sth, sph;
-          cart_to_bl(p.x - K.pos[0], p.y - K.pos[1], p.z - K.pos[2], K.a, sr, sth, sph);
-          out.steps = c;
-          out.dir2 = dir2;
-          out.seg_o = org1;
-          if (sr < K.Rhor) {
-            out.status = 2;
-          } else {
-            out.status = 1;
-            out.ent = ent;
-            out.prim = prim;
-            out.t = t;
-            out.ov = hs.ov;
-            out.ovc = hs.oc;
-            out.ove = hs.oe;
-          }
-          return;
-        }
-      }
-    }
-    if (far_mode) {
-      const float stf = sinf((float)y[1]);
-      if (stf * stf < (float)kPoleSin2) far_mode = false;  // a pole ahead: the reference's steps again
-    }
-    if (!far_mode) {
-      k.geodesic(y, dydx);
-      if (fabs(h_step) < 1.0e-10) {
-        out.status = 4;
-        out.steps = c;
-        out.dir2 = dir2;
-        return;
-      }
-    }
-    const double r_before = y[0];
-    if (capture_shortcut && !far_mode && !capture_checked && dydx[0] < 0.0 && y[0] < K.scene_inner) {
-      // inbound inside all scene geometry: captured if no turning point is
-      // left.  The reference ends such a ray with a step underflow (status 4)
-      // or inside the horizon (2); the shortcut reports 4, so it is taken only
-      // where the two look alike
-      capture_checked = true;
-      if (no_turning_point(y[0], rplus, K.a, k.L, k.kappa)) {
-        out.status = 4;
-        out.steps = c;
-        out.dir2 = dir2;
-        return;
-      }
-    }
-    for (int i = 0; i < 3; i++) yprev[i] = y[i];
-    if (far_mode) {
-      float yf[6], df[6], dy[6];
-#pragma unroll
-      for (int i = 0; i < 6; i++) yf[i] = (float)y[i];
-      kf.geodesic(yf, df);
-      kf.step(yf, df, (float)h_dist, dy);
-#pragma unroll
-      for (int i = 0; i < 6; i++) y[i] += (double)dy[i];
-      cnt.attempts++;
-      h_step = h_dist;
-    } else {
-      h_step = k.next_position(y, dydx, h_step, cnt.attempts, &errmax);
-      if (h_step > h_dist) h_step = h_dist;
-      if (y[0] < K.Rhor) {
-        out.status = 2;
-        out.steps = c;
-        out.dir2 = dir2;
-        return;
-      }
-      org1 = org2;
-      const dv3 q = bl_to_cart(y[0], y[1], y[2], K.a);
-      org2 = {q.x + K.pos[0], q.y + K.pos[1], q.z + K.pos[2]};
-      dir2 = dnormalize({org2.x - org1.x, org2.y - org1.y, org2.z - org1.z});
-      const double st = sin(y[1]);
-      if (y[0] > far && y[0] > r_before && errmax < kFarErrmax && h_step == h_dist && st * st >= kPoleSin2)
-        far_mode = true;
-    }
-    c++;
-    cnt.steps++;
-    if (K.escape_radius > 0.0 && y[0] > K.escape_radius && y[0] > r_before) break;
-  }
-  if (far_mode) {
+  double dydx[6];
+  M.k.initial(dir, M.y, dydx, r0, th0);
+  sincos(M.y[1], &M.sint, &M.cost);
+  M.h_step = kSegment;
+  M.errmax = 1.0;
+  M.org1 = M.org2 = org;
+  M.dir2 = dir;
+  for (int i = 0; i < 3; i++) M.yprev[i] = M.y[i];
+  M.c = 0;
+  M.far_mode = false;
+  M.capture_checked = false;
+  return true;
+}
+
+// The end of the loop: the polyline's last vertex looks straight on
+template <class HS>
+__device__ __forceinline__ void kerr_finish(const DevScene& S, const GKerr& K, KerrMarch& M, KerrHit& out,
+                                            KerrCount& cnt, uint32_t* err, HS& hs) {
+  if (M.far_mode) {
     // the polyline's last vertex and chord, in FP64, from the last two states
-    const dv3 q1 = bl_to_cart(yprev[0], yprev[1], yprev[2], K.a);
-    const dv3 q2 = bl_to_cart(y[0], y[1], y[2], K.a);
-    org2 = {q2.x + K.pos[0], q2.y + K.pos[1], q2.z + K.pos[2]};
-    dir2 = dnormalize({q2.x - q1.x, q2.y - q1.y, q2.z - q1.z});
+    const dv3 q1 = bl_to_cart(M.yprev[0], M.yprev[1], M.yprev[2], K.a);
+    const dv3 q2 = bl_to_cart(M.y[0], M.y[1], M.y[2], K.a);
+    M.org2 = {q2.x + K.pos[0], q2.y + K.pos[1], q2.z + K.pos[2]};
+    M.dir2 = dnormalize({q2.x - q1.x, q2.y - q1.y, q2.z - q1.z});
   }
-  out.steps = c;
-  out.dir2 = dir2;
-  out.seg_o = org2;
+  out.steps = M.c;
+  out.dir2 = M.dir2;
+  out.seg_o = M.org2;
   double t;
   int ent, prim;
   cnt.segments++;
-  if (exact_closest_hs(S, org2, dir2, t, ent, prim, err, cnt.nodes, cnt.tris, hs)) {
+  if (exact_closest_hs(S, M.org2, M.dir2, t, ent, prim, err, cnt.nodes, cnt.tris, hs)) {
     out.status = 5;
     out.ent = ent;
     out.prim = prim;
@@ -904,27 +734,236 @@ __device__ void kerr_trace_ray_fast(const DevScene& S, const GKerr& K, dv3 org, 
   }
 }
 
+// One pass of the reference's loop outside the far field, for the lanes that
+// run; true when the ray's trace has ended.  SYNC: all lanes of the warp call
+// it together, and the warp comes together again after the parts that few
+// lanes take.  look: with the segment test (not on the step that leaves the far field).
+template <bool FAST, bool SYNC, class HS>
+__device__ __forceinline__ bool kerr_step(const DevScene& S, const GKerr& K, KerrMarch& M, KerrHit& out,
+                                          KerrCount& cnt, uint32_t* err, HS& hs, bool capture_shortcut, bool run,
+                                          bool look) {
+  bool leave = run && M.c >= K.max_steps, done = false, hit = false;
+  double t = 0.0;
+  int ent = -1, prim = -1;
+  look = look && run && !leave;
+  int draws = 0;
+  if (look) draws = segment_draws(S, M.org1, M.dir2, kSegment, disk_alpha(K));
+  cnt.segments += look ? 1u : 0u;
+  for (int i = 0; i < draws; i++) (void)hs.rng->next();
+  if (draws < 0)  // the exact test makes its own draws
+    hit = exact_closest_hs(S, M.org1, M.dir2, t, ent, prim, err, cnt.nodes, cnt.tris, hs) && t < kSegment;
+  if (SYNC) __syncwarp();
+  if (hit) {
+    // hit point of intersect_scene_: (org1 + 1e-6 dir2) + t dir2
+    const dv3 o2 = dadd3(M.org1, dscale3(M.dir2, 0.000001));
+    const dv3 p = {o2.x + t * M.dir2.x, o2.y + t * M.dir2.y, o2.z + t * M.dir2.z};
+    double sr, sth, sph;
+    cart_to_bl(p.x - K.pos[0], p.y - K.pos[1], p.z - K.pos[2], K.a, sr, sth, sph);
+    out.steps = M.c;
+    out.dir2 = M.dir2;
+    out.seg_o = M.org1;
+    if (sr < K.Rhor) {
+      out.status = 2;
+    } else {
+      out.status = 1;
+      out.ent = ent;
+      out.prim = prim;
+      out.t = t;
+      out.ov = hs.ov;
+      out.ovc = hs.oc;
+      out.ove = hs.oe;
+    }
+    done = true;
+  } else if (run && !leave) {
+    double dydx[6];
+    M.k.geodesic(M.y, M.sint, M.cost, dydx);
+    if (fabs(M.h_step) < 1.0e-10) {
+      out.status = 4;
+      out.steps = M.c;
+      out.dir2 = M.dir2;
+      done = true;
+    }
+    if (FAST && !done) {
+      if (capture_shortcut && !M.capture_checked && dydx[0] < 0.0 && M.y[0] < K.scene_inner) {
+        // inbound inside all scene geometry: captured if no turning point is
+        // left.  The reference ends such a ray with a step underflow (status 4)
+        // or inside the horizon (2); the shortcut reports 4, so it is taken only
+        // where the two look alike
+        M.capture_checked = true;
+        if (no_turning_point(M.y[0], K.M + sqrt(K.M * K.M - K.a2), K.a, M.k.L, M.k.kappa)) {
+          out.status = 4;
+          out.steps = M.c;
+          out.dir2 = M.dir2;
+          done = true;
+        }
+      }
+      for (int i = 0; i < 3; i++) M.yprev[i] = M.y[i];
+    }
+    if (!done) {
+      const double r_before = M.y[0];
+      M.h_step = M.k.next_position(M.y, dydx, M.h_step, kSegment, cnt.attempts, &M.errmax);
+      if (M.y[0] < K.Rhor) {
+        out.status = 2;
+        out.steps = M.c;
+        out.dir2 = M.dir2;
+        done = true;
+      } else {
+        M.org1 = M.org2;
+        sincos(M.y[1], &M.sint, &M.cost);
+        const dv3 q = bl_to_cart(M.y[0], M.sint, M.cost, M.y[2], K.a);
+        M.org2 = {q.x + K.pos[0], q.y + K.pos[1], q.z + K.pos[2]};
+        M.dir2 = dnormalize({M.org2.x - M.org1.x, M.org2.y - M.org1.y, M.org2.z - M.org1.z});
+        if (FAST && M.y[0] > fmax(kFarRadius, K.scene_radius + 2.0) && M.y[0] > r_before && M.errmax < kFarErrmax &&
+            M.h_step == kSegment && M.sint * M.sint >= kPoleSin2)
+          M.far_mode = true;
+        M.c++;
+        cnt.steps++;
+        // optional early exit (not in the reference): far out and receding
+        leave = K.escape_radius > 0.0 && M.y[0] > K.escape_radius && M.y[0] > r_before;
+      }
+    }
+  }
+  if (SYNC) __syncwarp();
+  if (leave) {
+    kerr_finish(S, K, M, out, cnt, err, hs);
+    done = true;
+  }
+  return done;
+}
+
+// background map lookup of an escaped ray (scene.cpp:711-727; SphericalMapping::Map, circle.h:92-105)
+__device__ __forceinline__ float3 kerr_background(const GKerr& K, const double* yy, const float* bg) {
+  if (!K.texture) return f3(bg[0], bg[1], bg[2]);
+  double y1 = yy[1] * K.map_coef[0] + K.map_coef[1];
+  double y2 = yy[2] * K.map_coef[2] + K.map_coef[3];
+  y1 = fmod(y1, kPi);
+  y2 = fmod(y2, 2.0 * kPi);
+  double phi = y2, theta = y1;
+  if (phi < 0.0) phi += 2.0 * kPi;
+  if (theta < 0.0) theta = -theta;
+  int x = (int)(phi / (2.0 * kPi) * K.tex_w);
+  x = ((x % K.tex_w) + K.tex_w) % K.tex_w;  // in range for any input, NaN included
+  int yv = (int)(theta / kPi * K.tex_h);
+  yv = ((yv % K.tex_h) + K.tex_h) % K.tex_h;
+  const unsigned char* t = K.texture + 3 * ((size_t)yv * K.tex_w + x);
+  return f3((float)(K.texture_coef * t[0] / 255.0), (float)(K.texture_coef * t[1] / 255.0),
+            (float)(K.texture_coef * t[2] / 255.0));
+}
+
+template <class T>
+__device__ __forceinline__ T warp_sum(T v) {
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+  return v;
+}
+
+__device__ __forceinline__ void flush_counts(const KerrCount& c, uint32_t rays, unsigned long long* counters) {
+  if (!counters) return;
+  const unsigned long long a = warp_sum<unsigned long long>(rays), b = warp_sum<unsigned long long>(c.steps),
+                           d = warp_sum<unsigned long long>(c.attempts),
+                           e = warp_sum<unsigned long long>(c.segments);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(counters + 0, a);
+    atomicAdd(counters + 1, b);
+    atomicAdd(counters + 2, d);
+    atomicAdd(counters + 3, e);
+  }
+}
+
+
+// One step in the far field (FP32 increments to the FP64 state); true when
+// the ray's trace has ended.  A pole ahead ends the far field: then the step
+// is the reference's (kerr_step without its segment test).
+template <class HS>
+__device__ __forceinline__ bool kerr_far_step(const DevScene& S, const GKerr& K, KerrMarch& M, KerrHit& out,
+                                              KerrCount& cnt, uint32_t* err, HS& hs, bool capture_shortcut) {
+  if (M.c >= K.max_steps) {
+    kerr_finish(S, K, M, out, cnt, err, hs);
+    return true;
+  }
+  const float stf = sinf((float)M.y[1]);
+  if (stf * stf < (float)kPoleSin2) {
+    M.far_mode = false;
+    sincos(M.y[1], &M.sint, &M.cost);
+    return kerr_step<true, false>(S, K, M, out, cnt, err, hs, capture_shortcut, true, false);
+  }
+  const double r_before = M.y[0];
+  for (int i = 0; i < 3; i++) M.yprev[i] = M.y[i];
+  const KerrRayF kf{(float)K.a, (float)K.a2, (float)K.M, (float)M.k.L, (float)M.k.kappa};
+  float yf[6], df[6], dy[6];
+#pragma unroll
+  for (int i = 0; i < 6; i++) yf[i] = (float)M.y[i];
+  kf.geodesic(yf, df);
+  kf.step(yf, df, (float)kSegment, dy);
+#pragma unroll
+  for (int i = 0; i < 6; i++) M.y[i] += (double)dy[i];
+  cnt.attempts++;
+  M.h_step = kSegment;
+  M.c++;
+  cnt.steps++;
+  if (K.escape_radius > 0.0 && M.y[0] > K.escape_radius && M.y[0] > r_before) {
+    kerr_finish(S, K, M, out, cnt, err, hs);
+    return true;
+  }
+  return false;
+}
+
+// Rays of a batch (KerrOut), one per lane: a lane whose ray has ended takes
+// the next one
 template <bool FAST>
-__global__ void __launch_bounds__(128) kerr_trace_kernel(DevScene S, GKerr K, const double* __restrict__ rays,
-                                                         int64_t n, KerrOut out, uint32_t* __restrict__ err,
-                                                         unsigned long long* __restrict__ counters) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  KerrCount c{0, 0, 0, 0, 0};
-  uint32_t rays_done = 0;
-  if (i < n) {
+struct KerrTraceJob {
+  const DevScene& S;
+  const GKerr& K;
+  const double* rays;
+  int64_t n;
+  const KerrOut& out;
+  uint32_t* err;
+  unsigned long long* next;  // rays handed out beyond each lane's first
+  KerrMarch M;
+  KerrHit h;
+  KerrCount c;
+  Rng drng;
+  int64_t i;
+  uint32_t rays_done;
+  bool more, ended_at_start;
+
+  __device__ __forceinline__ bool take(bool want) {
+    const int lane = threadIdx.x & 31;
+    const unsigned int mask = __ballot_sync(0xffffffffu, want);
+    unsigned long long base = 0;
+    if (i < 0) {  // the first ray of every lane
+      base = (unsigned long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
+    } else {
+      const int leader = __ffs(mask) - 1;
+      if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(mask)) + (unsigned long long)gridDim.x * blockDim.x;
+      base = __shfl_sync(0xffffffffu, base, leader);
+    }
+    if (!want) return false;
+    i = (int64_t)(base + (unsigned long long)__popc(mask & ((1u << lane) - 1u)));
+    if (i >= n) {
+      more = false;
+      return false;
+    }
     const double* r = rays + 6 * i;
-    KerrHit h;
-    Rng drng;
     drng.init(disk_stream_key(0, K), (uint64_t)i, kDiskBranch);
+    if (!kerr_start(K, {r[0], r[1], r[2]}, {r[3], r[4], r[5]}, M, h)) ended_at_start = true;
+    return true;
+  }
+  __device__ __forceinline__ bool step(bool run) {
     KerrDiskShading hs{&K, &drng};
-    if (FAST) kerr_trace_ray_fast(S, K, {r[0], r[1], r[2]}, {r[3], r[4], r[5]}, h, c, err, hs, true);
-    else kerr_trace_ray(S, K, {r[0], r[1], r[2]}, {r[3], r[4], r[5]}, h, c, err, hs);
+    const bool far = FAST && run && M.far_mode && !ended_at_start;
+    bool done = run && ended_at_start;
+    done |= kerr_step<FAST, true>(S, K, M, h, c, err, hs, true, run && !far && !ended_at_start, true);
+    if (far) done = kerr_far_step(S, K, M, h, c, err, hs, true);
+    return done;
+  }
+  __device__ __forceinline__ bool ended() {
+    ended_at_start = false;
     if (out.status) out.status[i] = h.status;
     if (out.steps) out.steps[i] = h.steps;
     if (out.final_bl) {
-      out.final_bl[3 * i] = h.y[0];
-      out.final_bl[3 * i + 1] = h.y[1];
-      out.final_bl[3 * i + 2] = h.y[2];
+      out.final_bl[3 * i] = M.y[0];
+      out.final_bl[3 * i + 1] = M.y[1];
+      out.final_bl[3 * i + 2] = M.y[2];
     }
     if (out.exit_dir) {
       out.exit_dir[3 * i] = h.dir2.x;
@@ -933,128 +972,275 @@ __global__ void __launch_bounds__(128) kerr_trace_kernel(DevScene S, GKerr K, co
     }
     if (out.hit_entity) out.hit_entity[i] = h.ent;
     if (out.hit_t) out.hit_t[i] = h.t;
-    rays_done = 1;
-  }
-  flush_counts(c, rays_done, counters);
-}
-
-// A closest-hit query of the renderer along a geodesic: on a hit, the vertex
-// the straight-ray tracer would build from the last segment; on a miss, the
-// colour radiance() returns (horizon black, background map or BACKGROUND).
-template <bool FAST>
-__device__ bool kerr_closest(const DevScene& S, const GKerr& K, float3 o, float3 d, FastHit& h, Vertex& v,
-                             float3& miss, float3 ovr[2], bool& has_ovr, KerrCount& c, uint32_t* err, Rng& drng) {
-  KerrHit k;
-  KerrDiskShading hs{&K, &drng};
-  // a captured ray's colour: black (horizon) or BACKGROUND (step underflow)
-  // are the same only on a black background
-  const bool black_bg = S.bg[0] == 0.0f && S.bg[1] == 0.0f && S.bg[2] == 0.0f;
-  if (FAST) kerr_trace_ray_fast(S, K, {o.x, o.y, o.z}, {d.x, d.y, d.z}, k, c, err, hs, black_bg);
-  else kerr_trace_ray(S, K, {o.x, o.y, o.z}, {d.x, d.y, d.z}, k, c, err, hs);
-  has_ovr = false;
-  if (k.status != 1) {
-    if (k.status == 2) miss = f3(0, 0, 0);
-    else if (k.status == 0) miss = kerr_background(K, k.y, S.bg);
-    else miss = f3(S.bg[0], S.bg[1], S.bg[2]);
+    rays_done++;
     return false;
   }
-  const GEntity& e = S.ents[k.ent];
-  const dv3 o2 = dadd3(k.seg_o, dscale3(k.dir2, 0.000001));
-  const dv3 p = {o2.x + k.t * k.dir2.x, o2.y + k.t * k.dir2.y, o2.z + k.t * k.dir2.z};
-  float3 n;
-  if (e.type == PR_ENT_SPHERE) {
-    n = normalize(f3((float)(p.x - e.p[0]), (float)(p.y - e.p[1]), (float)(p.z - e.p[2])));
-  } else if (e.type == PR_ENT_POLYGON) {
-    n = ld3(S.fnorm + 3 * (size_t)(e.face_base + k.prim));
-  } else {
-    n = f3((float)e.normal[0], (float)e.normal[1], (float)e.normal[2]);
-  }
-  if (e.normal_inverse < 0) n = -n;
-  v.p = f3((float)p.x, (float)p.y, (float)p.z);
-  v.n = n;
-  v.ent = k.ent;
-  v.mat = e.material;
-  v.t = (float)k.t;
-  if (k.ov) {  // the accretion disk's own colour and emission at this point
-    has_ovr = true;
-    ovr[0] = k.ovc;
-    ovr[1] = k.ove;
-  }
-  h.t = (float)k.t;
-  h.ent = k.ent;
-  h.slot = -1;
-  h.u = h.v = 0.0f;
-  return true;
+};
+
+template <bool FAST>
+__global__ void __launch_bounds__(128) kerr_trace_kernel(const __grid_constant__ DevScene S,
+                                                         const __grid_constant__ GKerr K,
+                                                         const double* __restrict__ rays, int64_t n,
+                                                         const __grid_constant__ KerrOut out,
+                                                         uint32_t* __restrict__ err,
+                                                         unsigned long long* __restrict__ counters) {
+  KerrTraceJob<FAST> job{S, K, rays, n, out, err, counters + kKerrNextCounter};
+  job.c = KerrCount{0, 0, 0, 0, 0};
+  job.i = -1;
+  job.rays_done = 0;
+  job.more = true;
+  job.ended_at_start = false;
+  geodesic_warp(job);
+  flush_counts(job.c, job.rays_done, counters);
 }
 
-// one camera sample of radiance() in a Kerr scene (no next-event estimation,
-// no media: every query is a geodesic, as intersect_scene makes it)
-template <bool FAST>
-__device__ float3 kerr_trace_sample(const DevScene& S, const GKerr& K, const RenderCfg& cfg, float3 o0, float3 d0,
-                                    uint64_t sample_id, KerrCount& c, uint32_t* err) {
-  PathState stack[kSplitStack];
-  int sp = 0;
-  root_path(stack[sp++], o0, d0);
-  float3 L = f3(0, 0, 0);
+// A path in the far field, handed from the near kernel of the mixed form to
+// the far one
+struct KerrFar {
+  double y[6], yprev[3], L, kappa, h_step, errmax;
+  dv3 org2, dir2;
+  unsigned long long id;
+  Rng drng;
+  PathState ps;
+  float3 root;
+  int c;
+  int capture_checked;
+};
+
+struct KerrFrame {
+  long long* pix;              // 3 per pixel, fixed point (kPixelScaleF)
+  unsigned long long* next;    // [0] samples handed out, [1] far records written, [2] far records taken
+  unsigned long long samples;  // of the frame
+  KerrFar* far;                // mixed form
+  unsigned long long far_cap;
+};
+
+// Camera samples of radiance() in a Kerr scene, one path per lane (no
+// next-event estimation, no media: every query is a geodesic, as
+// intersect_scene makes it).  PHASE 0: the FP64 form; 1: the mixed form's
+// near field, which hands a path that reaches the far field on; 2: its far
+// field, from those records.  A step near the hole costs the FP64 pipe what
+// fifty far steps cost the FP32 ones; side by side in a warp each waited for
+// the other.
+template <int PHASE>
+struct KerrPathJob {
+  static constexpr bool FAST = PHASE != 0;
+  const DevScene& S;
+  const GKerr& K;
+  const RenderCfg& cfg;
+  const KerrFrame& F;
+  uint32_t* err;
+  KerrMarch M;
+  KerrHit h;
+  KerrCount c;
   Rng drng;  // the accretion disk's alpha tests of this camera sample
-  drng.init(disk_stream_key(cfg.seed, K), sample_id, kDiskBranch);
-  while (sp > 0) {
-    PathState ps = stack[--sp];
-    for (;;) {
-      FastHit h;
-      Vertex v;
-      float3 miss, ovr[2];
-      bool has_ovr;
-      const bool hit = kerr_closest<FAST>(S, K, ps.o, ps.d, h, v, miss, ovr, has_ovr, c, err, drng);
-      ShadowReq sh[3];
-      int nsh = 0;
-      PathState child;
-      const int r = shade(S, cfg, ps, hit, h, sample_id, sh, nsh, child, err, &v, &miss, nullptr, nullptr,
-                          has_ovr ? ovr : nullptr);
-      if (r == SHADE_SPLIT) {
-        if (sp < kSplitStack) stack[sp++] = child;
-        else atomicOr(err, PR_DEV_LOOP_CAP);
-      }
-      if (r == SHADE_END) break;
-    }
-    L += ps.L;
-  }
-  return L;
-}
+  PathState ps;
+  unsigned long long id;
+  float3 L;
+  int sp;
+  uint32_t paths;
+  bool more, ended_at_start;
+  PathState stack[kSplitStack];
 
-template <bool FAST>
-__global__ void __launch_bounds__(128) kerr_render_kernel(DevScene S, GKerr K, RenderCfg cfg, float* __restrict__ out,
+  // a captured ray's colour: black (horizon) or BACKGROUND (step underflow)
+  // are the same only on a black background
+  __device__ __forceinline__ bool shortcut() const { return S.bg[0] == 0.0f && S.bg[1] == 0.0f && S.bg[2] == 0.0f; }
+
+  __device__ __forceinline__ void start_ray() {
+    ended_at_start = !kerr_start(K, {ps.o.x, ps.o.y, ps.o.z}, {ps.d.x, ps.d.y, ps.d.z}, M, h);
+  }
+
+  __device__ __forceinline__ bool take(bool want) {
+    const int lane = threadIdx.x & 31;
+    const unsigned int mask = __ballot_sync(0xffffffffu, want);
+    const int leader = __ffs(mask) - 1;
+    unsigned long long base = 0;
+    if (lane == leader) base = atomicAdd(F.next + (PHASE == 2 ? 2 : 0), (unsigned long long)__popc(mask));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (!want) return false;
+    const unsigned long long g = base + (unsigned long long)__popc(mask & ((1u << lane) - 1u));
+    sp = 0;
+    if (PHASE == 2) {
+      const unsigned long long n = F.next[1] < F.far_cap ? F.next[1] : F.far_cap;
+      if (g >= n) {
+        more = false;
+        return false;
+      }
+      const KerrFar& f = F.far[g];
+      for (int q = 0; q < 6; q++) M.y[q] = f.y[q];
+      for (int q = 0; q < 3; q++) M.yprev[q] = f.yprev[q];
+      M.k = KerrRay{K.a, K.a2, K.M, f.L, f.kappa};
+      M.h_step = f.h_step;
+      M.errmax = f.errmax;
+      M.org1 = M.org2 = f.org2;
+      M.dir2 = f.dir2;
+      M.c = f.c;
+      M.far_mode = true;
+      M.capture_checked = f.capture_checked != 0;
+      M.sint = M.cost = 0.0;
+      h.steps = 0;
+      h.ov = false;
+      h.ent = -1;
+      h.prim = -1;
+      h.t = -1.0;
+      id = f.id;
+      drng = f.drng;
+      ps = f.ps;
+      L = f.root;
+      ended_at_start = false;
+      return true;
+    }
+    if (g >= F.samples) {
+      more = false;
+      return false;
+    }
+    const unsigned long long px = g / (unsigned int)cfg.spp;
+    const uint32_t k = (uint32_t)(g - px * (unsigned int)cfg.spp);
+    const int y = (int)((uint32_t)px / (uint32_t)cfg.width), x = (int)((uint32_t)px - (uint32_t)y * cfg.width);
+    float3 o, d;
+    id = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
+    root_path(ps, o, d);
+    drng.init(disk_stream_key(cfg.seed, K), id, kDiskBranch);
+    L = f3(0, 0, 0);
+    start_ray();
+    return true;
+  }
+
+  __device__ __forceinline__ bool step(bool run) {
+    KerrDiskShading hs{&K, &drng};
+    const bool far = FAST && run && M.far_mode && !ended_at_start;
+    bool done = run && ended_at_start;
+    done |= kerr_step<FAST, true>(S, K, M, h, c, err, hs, FAST && shortcut(), run && !far && !ended_at_start, true);
+    if (PHASE == 1) {
+      // newly in the far field (or started a step there: no room in the list)
+      if (run && !done && M.far_mode) {
+        unsigned long long at = F.far_cap;
+        if (!far && sp == 0) at = atomicAdd(F.next + 1, 1ull);
+        if (at < F.far_cap) {
+          KerrFar& f = F.far[at];
+          for (int q = 0; q < 6; q++) f.y[q] = M.y[q];
+          for (int q = 0; q < 3; q++) f.yprev[q] = M.yprev[q];
+          f.L = M.k.L;
+          f.kappa = M.k.kappa;
+          f.h_step = M.h_step;
+          f.errmax = M.errmax;
+          f.org2 = M.org2;
+          f.dir2 = M.dir2;
+          f.c = M.c;
+          f.capture_checked = M.capture_checked;
+          f.id = id;
+          f.drng = drng;
+          f.ps = ps;
+          f.root = L;
+          h.status = -1;  // handed on
+          done = true;
+        }
+      }
+    }
+    if (far) done = kerr_far_step(S, K, M, h, c, err, hs, shortcut());
+    return done;
+  }
+
+  // the ray's trace ended: shade, and go on with the path's next ray or end it
+  __device__ __forceinline__ bool ended() {
+    if (PHASE == 1 && h.status == -1) return false;
+    FastHit fh;
+    Vertex v;
+    float3 miss = f3(0, 0, 0), ovr[2];
+    bool has_ovr = false;
+    const bool hit = h.status == 1;
+    if (!hit) {
+      if (h.status == 0) miss = kerr_background(K, M.y, S.bg);
+      else if (h.status != 2) miss = f3(S.bg[0], S.bg[1], S.bg[2]);
+    } else {
+      // the vertex the straight-ray tracer would build from the last segment
+      const GEntity& e = S.ents[h.ent];
+      const dv3 o2 = dadd3(h.seg_o, dscale3(h.dir2, 0.000001));
+      const dv3 p = {o2.x + h.t * h.dir2.x, o2.y + h.t * h.dir2.y, o2.z + h.t * h.dir2.z};
+      float3 n;
+      if (e.type == PR_ENT_SPHERE) {
+        n = normalize(f3((float)(p.x - e.p[0]), (float)(p.y - e.p[1]), (float)(p.z - e.p[2])));
+      } else if (e.type == PR_ENT_POLYGON) {
+        n = ld3(S.fnorm + 3 * (size_t)(e.face_base + h.prim));
+      } else {
+        n = f3((float)e.normal[0], (float)e.normal[1], (float)e.normal[2]);
+      }
+      if (e.normal_inverse < 0) n = -n;
+      v.p = f3((float)p.x, (float)p.y, (float)p.z);
+      v.n = n;
+      v.ent = h.ent;
+      v.mat = e.material;
+      v.t = (float)h.t;
+      if (h.ov) {  // the accretion disk's own colour and emission at this point
+        has_ovr = true;
+        ovr[0] = h.ovc;
+        ovr[1] = h.ove;
+      }
+      fh.t = (float)h.t;
+      fh.ent = h.ent;
+      fh.slot = -1;
+      fh.u = fh.v = 0.0f;
+    }
+    ShadowReq sh[3];
+    int nsh = 0;
+    PathState child;
+    const int r = shade(S, cfg, ps, hit, fh, id, sh, nsh, child, err, &v, &miss, nullptr, nullptr,
+                        has_ovr ? ovr : nullptr);
+    if (r == SHADE_SPLIT) {
+      if (sp < kSplitStack) stack[sp++] = child;
+      else atomicOr(err, PR_DEV_LOOP_CAP);
+    }
+    if (r == SHADE_END) {
+      L += ps.L;
+      if (sp == 0) {
+        const float3 val = finish_sample(cfg, L, err);
+        const uint32_t p = (uint32_t)(id % ((unsigned long long)cfg.width * cfg.height));
+        const uint32_t y = p / (uint32_t)cfg.width, x = p - y * (uint32_t)cfg.width;
+        add_pixel(F.pix + 3 * ((size_t)(cfg.height - 1 - y) * cfg.width + x), val);
+        paths++;
+        return false;
+      }
+      ps = stack[--sp];
+    }
+    start_ray();
+    return true;
+  }
+};
+
+template <int PHASE>
+__global__ void __launch_bounds__(128) kerr_render_kernel(const __grid_constant__ DevScene S,
+                                                          const __grid_constant__ GKerr K,
+                                                          const __grid_constant__ RenderCfg cfg,
+                                                          const __grid_constant__ KerrFrame F,
                                                           uint32_t* __restrict__ err,
                                                           unsigned long long* __restrict__ counters) {
-  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t warp = tid >> 5, lane = tid & 31;
-  const uint32_t tiles_per_chunk = cfg.tiles_x * cfg.tiles_y;
-  const uint32_t chunk = warp / tiles_per_chunk;
-  if (chunk >= (uint32_t)cfg.chunks) return;
-  const uint32_t tile = warp - chunk * tiles_per_chunk;
-  const int x = (int)((tile % cfg.tiles_x) * 8 + (lane & 7));
-  const int y = (int)((tile / cfg.tiles_x) * 4 + (lane >> 3));
-  KerrCount c{0, 0, 0, 0, 0};
-  uint32_t paths = 0;
-  if (x < cfg.width && y < cfg.height) {
-    const int k0 = (int)(((int64_t)cfg.spp * chunk) / cfg.chunks);
-    const int k1 = (int)(((int64_t)cfg.spp * (chunk + 1)) / cfg.chunks);
-    float3 acc = f3(0, 0, 0);
-    for (int k = k0; k < k1; k++) {
-      float3 o, d;
-      const uint64_t sample_id = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
-      acc += finish_sample(cfg, kerr_trace_sample<FAST>(S, K, cfg, o, d, sample_id, c, err), err);
-      paths++;
-    }
-    acc = acc * cfg.sensor;
-    float* po = out + 3 * ((size_t)chunk * cfg.width * cfg.height + (size_t)(cfg.height - y - 1) * cfg.width + x);
-    po[0] = acc.x;
-    po[1] = acc.y;
-    po[2] = acc.z;
-  }
-  flush_counts(c, paths, counters);
+  KerrPathJob<PHASE> job{S, K, cfg, F, err};
+  job.c = KerrCount{0, 0, 0, 0, 0};
+  job.sp = 0;
+  job.paths = 0;
+  job.more = true;
+  job.ended_at_start = false;
+  geodesic_warp(job);
+  flush_counts(job.c, job.paths, counters);
 }
 
+// scratch of a frame: the pixel sums and counters (zeroed), the far records
+inline size_t kerr_zero_bytes(const RenderCfg& cfg) {
+  return (24 * (size_t)cfg.width * cfg.height + 32 + 255) / 256 * 256;
+}
+inline unsigned long long kerr_far_cap(const RenderCfg& cfg) {
+  const unsigned long long n = (unsigned long long)cfg.spp * cfg.width * cfg.height;
+  return n < (1ull << 19) ? n : 1ull << 19;  // beyond that the near kernel goes on itself
+}
+inline KerrFrame kerr_frame(const RenderCfg& cfg, void* scratch, bool far) {
+  KerrFrame F;
+  F.pix = static_cast<long long*>(scratch);
+  F.next = reinterpret_cast<unsigned long long*>(F.pix + 3 * (size_t)cfg.width * cfg.height);
+  F.samples = (unsigned long long)cfg.spp * cfg.width * cfg.height;
+  F.far = far ? reinterpret_cast<KerrFar*>(static_cast<char*>(scratch) + kerr_zero_bytes(cfg)) : nullptr;
+  F.far_cap = far ? kerr_far_cap(cfg) : 0;
+  return F;
+}
 
 }  // namespace
 }  // namespace pr

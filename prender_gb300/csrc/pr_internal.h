@@ -159,7 +159,9 @@ struct GEntF {
   float sss_rmax;  // subsurface probe-disk radius for this object (its bounding-box clamp applied)
   int32_t light_id;  // lights: registration index (Entity::light_id), which the reference
                      // uses as an index into the sorted list (directLight_radiance.h:541)
-  // disk: u_length = radius, v_length = inner radius, n = the plane normal
+  // disk: u_length = radius, v_length = inner radius, n = the plane normal,
+  // u / v the base plane's axes over their lengths, node_base: an accretion
+  // disk whose alpha test draws
   // sphere: the FP32 bounds' anchor u, q = anchor - centre (high parts v, low
   // parts n), c0 = |q|^2 - r^2 (high u_length, low v_length) and node_base =
   // hemisphere (trace_fast.cuh)
@@ -236,6 +238,7 @@ struct GKerr {
   int32_t use_temp;              // use_accretion_disk_temperature
   int32_t pad0;
   uint64_t disk_seed;            // key of the alpha-test stream
+  float rms_f, a2_f, pos_f[3];   // FP32 copies (geodesic_math.cuh)
 };
 
 // Everything a kernel needs, passed by value (fits the 4 KB param space).

@@ -182,9 +182,6 @@ __global__ void reduce_chunks(const float* __restrict__ partial, float* __restri
 // (block_paths.cuh), and add each finished sample to its pixel in 64-bit
 // fixed point (2^-40: integer sums do not depend on the order in which
 // samples finish).
-constexpr float kPixelScaleF = 1099511627776.0f;  // 2^40
-constexpr float kPixelInvF = 1.0f / 1099511627776.0f;
-
 struct PlainFrame {
   long long* pix;              // 3 per pixel
   unsigned long long* next;    // samples handed out
@@ -274,11 +271,7 @@ struct PlainPaths {
     const float3 v = finish_sample(cfg, L, err);
     const uint32_t p = (uint32_t)(id % ((unsigned long long)cfg.width * cfg.height));
     const uint32_t y = p / (uint32_t)cfg.width, x = p - y * (uint32_t)cfg.width;
-    unsigned long long* px =
-        reinterpret_cast<unsigned long long*>(F.pix + 3 * ((size_t)(cfg.height - 1 - y) * cfg.width + x));
-    atomicAdd(px + 0, (unsigned long long)__float2ll_rn(v.x * kPixelScaleF));
-    atomicAdd(px + 1, (unsigned long long)__float2ll_rn(v.y * kPixelScaleF));
-    atomicAdd(px + 2, (unsigned long long)__float2ll_rn(v.z * kPixelScaleF));
+    add_pixel(F.pix + 3 * ((size_t)(cfg.height - 1 - y) * cfg.width + x), v);
     paths++;
     return SHADE_END;
   }
@@ -305,6 +298,11 @@ __global__ void resolve_pixels(const long long* __restrict__ pix, float* __restr
   if (i >= n3) return;
   const float v = __ll2float_rn(pix[i]) * kPixelInvF * sensor;
   dst[i] = accumulate ? dst[i] + v : v;
+}
+
+cudaError_t launch_resolve(const long long* pix, float* dst, int n3, int accumulate, float sensor, cudaStream_t stream) {
+  resolve_pixels<<<(n3 + 255) / 256, 256, 0, stream>>>(pix, dst, n3, accumulate, sensor);
+  return cudaGetLastError();
 }
 
 // scratch: the pixel sums and the sample counter (zeroed by the launch), then the pool
@@ -335,8 +333,7 @@ cudaError_t launch_plain(const DevScene& S, const RenderCfg& cfg, void* scratch,
     pt_block<false><<<b.blocks, b.threads, smem, stream>>>(S, cfg, F, P, err, counters);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  resolve_pixels<<<(unsigned int)((n3 + 255) / 256), 256, 0, stream>>>(F.pix, dst, (int)n3, accumulate, cfg.sensor);
-  return cudaGetLastError();
+  return launch_resolve(F.pix, dst, (int)n3, accumulate, cfg.sensor, stream);
 }
 
 cudaError_t launch_megakernel(const DevScene& S, const RenderCfg& cfg, float* out, uint32_t* err,

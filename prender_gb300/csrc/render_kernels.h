@@ -27,6 +27,29 @@ struct RenderCfg {
   uint64_t sample_offset;
 };
 
+// Pixel sums in 64-bit fixed point (2^-40): integer sums do not depend on the
+// order in which samples finish.
+constexpr float kPixelScaleF = 1099511627776.0f;  // 2^40
+constexpr float kPixelInvF = 1.0f / 1099511627776.0f;
+#ifdef __CUDACC__
+__device__ __forceinline__ void add_pixel(long long* pix, float3 v) {
+  unsigned long long* p = reinterpret_cast<unsigned long long*>(pix);
+  atomicAdd(p + 0, (unsigned long long)__float2ll_rn(v.x * kPixelScaleF));
+  atomicAdd(p + 1, (unsigned long long)__float2ll_rn(v.y * kPixelScaleF));
+  atomicAdd(p + 2, (unsigned long long)__float2ll_rn(v.z * kPixelScaleF));
+}
+#endif
+// pixel sums -> float image times the sensor response; accumulate adds to it
+cudaError_t launch_resolve(const long long* pix, float* dst, int n3, int accumulate, float sensor, cudaStream_t stream);
+// SMs of the current device
+inline int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    sms = 152;
+  return sms;
+}
+
 cudaError_t launch_megakernel(const DevScene& S, const RenderCfg& cfg, float* out, uint32_t* err,
                               unsigned long long* counters, cudaStream_t stream);
 cudaError_t launch_reduce(const float* partial, float* dst, int n3, int chunks, int accumulate, cudaStream_t stream);

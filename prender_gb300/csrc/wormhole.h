@@ -22,9 +22,10 @@ struct WormOut {
 cudaError_t launch_worm_trace(const DevScene& S, const GWorm& W, const double* rays, int64_t n, WormOut out,
                               uint32_t* err, unsigned long long* counters, cudaStream_t stream);
 
-// the renderer with every scene query traced through the wormhole; same
-// output layout as launch_megakernel (per-chunk partial images)
-cudaError_t launch_worm_render(const DevScene& S, const GWorm& W, const RenderCfg& cfg, float* partial, uint32_t* err,
-                               unsigned long long* counters, cudaStream_t stream);
+// the renderer with every scene query traced through the wormhole, into dst
+// (scratch of worm_scratch_bytes): a kernel and the resolve
+size_t worm_scratch_bytes(const RenderCfg& cfg);
+cudaError_t launch_worm_render(const DevScene& S, const GWorm& W, const RenderCfg& cfg, void* scratch, float* dst,
+                               int accumulate, uint32_t* err, unsigned long long* counters, cudaStream_t stream);
 
 }  // namespace pr
