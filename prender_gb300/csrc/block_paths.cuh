@@ -184,7 +184,7 @@ __device__ __forceinline__ void block_paths(const DevScene& S, const BlockPool& 
   for (int s = tid; s < P.slots; s += nt) alive[s] = 0;
   // a small frame's slots go to the warps in turn
   const int warps = nt / 32;
-  const bool spread = P.slots_used < nt;
+  const bool spread = 2 * P.slots_used <= nt;
   for (unsigned int guard = 0;; guard++) {
     __syncthreads();
     if (tid == 0) {

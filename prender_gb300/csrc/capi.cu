@@ -116,7 +116,8 @@ void pr_destroy(pr_ctx* c) {
                     &c->wf_L, &c->wf_sample, &c->wf_hit, &c->wf_hitv, &c->wf_nee, &c->wf_sho, &c->wf_shd, &c->wf_extq,
                     &c->wf_shq, &c->wf_spo, &c->wf_spd, &c->wf_spb, &c->wf_spw, &c->wf_sps, &c->wf_samp, &c->wf_live,
                     &c->wf_pix, &c->wf_ctl, &c->wf_frc, &c->wf_fre, &c->wf_frs, &c->wf_frl, &c->wf_spf,
-                    &c->wf_neef})
+                    &c->wf_neef, &c->mlt_lum, &c->mlt_path, &c->mlt_start, &c->mlt_u, &c->mlt_cur, &c->mlt_acc,
+                    &c->mlt_slots})
     b->release();
   if (c->wf_graph) cudaGraphExecDestroy(c->wf_graph);
   if (c->batch_exec) cudaGraphExecDestroy(c->batch_exec);
@@ -696,7 +697,7 @@ static unsigned int wavefront_slots() {
 // bootstrap of samples x (int)(W H pre_sample) paths on the GPU, their
 // luminances read back for b and for the chains' starts (systematic
 // resampling in proportion to luminance), then samples x (int)(W H
-// mutation) mutations spread over the chains in launches of a few
+// mutation) mutations spread over the chains in launches of some
 // iterations; the image is the chains' mean times the sensor response / 4.
 static int render_mlt(pr_ctx* c, const RenderCfg& g0, const pr_render_params* p, float* rgb_dev, int accumulate,
                       uint64_t& paths_out, uint64_t& launches_out) {
@@ -726,11 +727,13 @@ static int render_mlt(pr_ctx* c, const RenderCfg& g0, const pr_render_params* p,
   PR_CUDA(c, c->mlt_u.ensure(sizeof(float) * (size_t)m.chains * kMltDims));
   PR_CUDA(c, c->mlt_cur.ensure(sizeof(float4) * (size_t)m.chains));
   PR_CUDA(c, c->mlt_acc.ensure(sizeof(float) * n3));
+  PR_CUDA(c, c->mlt_slots.ensure(mlt_scratch_bytes(m)));
   PR_CUDA(c, cudaMemsetAsync(c->mlt_acc.p, 0, sizeof(float) * n3, c->stream));
   const DevScene& S = c->cur.dev;
   uint32_t* err = (uint32_t*)c->errword.p;
   unsigned long long* cnt = (unsigned long long*)c->counters.p;
-  PR_CUDA(c, launch_mlt_seeds(S, g, m, (float*)c->mlt_lum.p, (float4*)c->mlt_path.p, err, cnt, c->stream));
+  PR_CUDA(c, launch_mlt_seeds(S, g, m, (float*)c->mlt_lum.p, (float4*)c->mlt_path.p, c->mlt_slots.p, err, cnt,
+                              c->stream));
   std::vector<float> lum((size_t)m.seeds);
   PR_CUDA(c, cudaMemcpyAsync(lum.data(), c->mlt_lum.p, sizeof(float) * lum.size(), cudaMemcpyDeviceToHost, c->stream));
   PR_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -752,10 +755,12 @@ static int render_mlt(pr_ctx* c, const RenderCfg& g0, const pr_render_params* p,
                                c->stream));
     PR_CUDA(c, launch_mlt_init(m, (const int32_t*)c->mlt_start.p, (const float4*)c->mlt_path.p,
                                (const float*)c->mlt_lum.p, (float*)c->mlt_u.p, (float4*)c->mlt_cur.p, c->stream));
-    const int64_t per_launch = 8;
+    // a launch ends with its longest paths on an emptying chip: 64 iterations
+    // each instead of 8
+    const int64_t per_launch = 64;
     for (int64_t it = 0; it < m.mutations; it += per_launch)
       PR_CUDA(c, launch_mlt_chains(S, g, m, it, std::min<int64_t>(m.mutations, it + per_launch), (float*)c->mlt_u.p,
-                                   (float4*)c->mlt_cur.p, (float*)c->mlt_acc.p, err, cnt, c->stream));
+                                   (float4*)c->mlt_cur.p, (float*)c->mlt_acc.p, c->mlt_slots.p, err, cnt, c->stream));
     paths_out += (uint64_t)m.chains * (uint64_t)m.mutations;
     launches_out += 1 + (uint64_t)((m.mutations + per_launch - 1) / per_launch);
   }

@@ -64,7 +64,7 @@ struct pr_ctx {
   pr::DevBuf partial, out, rays, ires, jres, dres;
   pr::DevBuf k_status, k_bl, k_dir, k_steps, k_ent, k_t;  // pr_kerr_trace staging
   pr::DevBuf k_sens;                                        // pr_kerr_sensitivity staging
-  pr::DevBuf mlt_lum, mlt_path, mlt_start, mlt_u, mlt_cur, mlt_acc;  // PR_MODE_MLT state
+  pr::DevBuf mlt_lum, mlt_path, mlt_start, mlt_u, mlt_cur, mlt_acc, mlt_slots;  // PR_MODE_MLT state
   pr::DevBuf adj_scratch, adj_grad;                         // adjoint outputs
   pr::DevBuf adj_samples;                                   // a pass's samples and path slots
   double kernel_ms[4] = {0, 0, 0, 0};        // wavefront shade / extend / shadow / control (host-driven loop)

@@ -13,7 +13,7 @@ namespace pr {
 constexpr int kMltDims = 64;
 
 struct MltCfg {
-  int chains;            // independent Markov chains (one thread each)
+  int chains;            // independent Markov chains
   int seeds;             // bootstrap paths
   int64_t mutations;     // per chain
   float b;               // mean luminance of the bootstrap paths
@@ -23,10 +23,12 @@ struct MltCfg {
   uint64_t seed;
 };
 
+// scratch of the launches below
+size_t mlt_scratch_bytes(const MltCfg& m);
 // bootstrap: seeds paths from fresh primary samples -> luminance, colour
 // and pixel of each
 cudaError_t launch_mlt_seeds(const DevScene& S, const RenderCfg& cfg, const MltCfg& m, float* lum, float4* path,
-                             uint32_t* err, unsigned long long* counters, cudaStream_t stream);
+                             void* scratch, uint32_t* err, unsigned long long* counters, cudaStream_t stream);
 // chains start from start[c] (a bootstrap index): primary samples and the
 // current path's colour / pixel / luminance
 cudaError_t launch_mlt_init(const MltCfg& m, const int32_t* start, const float4* seed_path, const float* seed_lum,
@@ -35,8 +37,8 @@ cudaError_t launch_mlt_init(const MltCfg& m, const int32_t* start, const float4*
 // proposed path with Kelemen's weights into acc (3 floats per pixel),
 // accept or keep
 cudaError_t launch_mlt_chains(const DevScene& S, const RenderCfg& cfg, const MltCfg& m, int64_t it0, int64_t it1,
-                              float* u, float4* cur, float* acc, uint32_t* err, unsigned long long* counters,
-                              cudaStream_t stream);
+                              float* u, float4* cur, float* acc, void* scratch, uint32_t* err,
+                              unsigned long long* counters, cudaStream_t stream);
 // rgb (+)= acc * scale
 cudaError_t launch_mlt_resolve(const float* acc, float* rgb, int n3, float scale, int accumulate, cudaStream_t stream);
 
