@@ -48,7 +48,7 @@ __device__ __forceinline__ void frame_release(SssFrames& F, float3& root, int f)
 }
 
 // One camera sample: the whole branch tree of radiance() for one root ray.
-template <bool SSS>
+template <bool SSS, bool EXT>
 __device__ float3 trace_sample(const DevScene& S, const RenderCfg& cfg, float3 o0, float3 d0, uint64_t sample_id,
                                TraceStats& st, uint32_t* err, uint32_t& segs) {
   PathState stack[kSplitStack];
@@ -73,7 +73,7 @@ __device__ float3 trace_sample(const DevScene& S, const RenderCfg& cfg, float3 o
       SssFrameOut fo;
       fo.open = 0;
       const float3 Lb = ps.L;
-      const int r = shade<SSS, SSS, SSS>(S, cfg, ps, hit, h, sample_id, sh, nsh, child, err, nullptr, nullptr,
+      const int r = shade<SSS, EXT, EXT>(S, cfg, ps, hit, h, sample_id, sh, nsh, child, err, nullptr, nullptr,
                                          nullptr, SSS ? &fo : nullptr);
       const float3 Lown = ps.L - Lb;
       float3 Lnee = f3(0, 0, 0);
@@ -134,8 +134,8 @@ __device__ float3 trace_sample(const DevScene& S, const RenderCfg& cfg, float3 o
 // the lean form (no subsurface or glossy lobes) at 8 blocks of 128 per SM
 // (64 registers, spilling): plain mesh Cornell box 23.6 -> 24.8 Mpaths/s
 // on GB300; the fuller form keeps 3 blocks per SM (168 registers)
-template <bool SSS>
-__global__ void __launch_bounds__(128, SSS ? 3 : 8) pt_megakernel(DevScene S, RenderCfg cfg, float* __restrict__ out,
+template <bool SSS, bool EXT>
+__global__ void __launch_bounds__(128, EXT ? 3 : 8) pt_megakernel(DevScene S, RenderCfg cfg, float* __restrict__ out,
                                                      uint32_t* __restrict__ err, unsigned long long* __restrict__ counters) {
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t warp = tid >> 5, lane = tid & 31;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(128, SSS ? 3 : 8) pt_megakernel(DevScene S, Re
     for (int k = k0; k < k1; k++) {
       float3 o, d;
       const uint64_t sample_id = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
-      acc += finish_sample(cfg, trace_sample<SSS>(S, cfg, o, d, sample_id, st, err, segs), err);
+      acc += finish_sample(cfg, trace_sample<SSS, EXT>(S, cfg, o, d, sample_id, st, err, segs), err);
       paths++;
     }
     acc = acc * cfg.sensor;
@@ -237,12 +237,7 @@ struct PlainPaths {
                                         ShadowReq* sh, int& nsh) {
     PathState child;
     const unsigned long long id = P.id[i];
-    // FULL: the per-thread form's fuller instantiation itself (its subsurface
-    // case is not reached), so that both round alike
-    SssFrameOut fo;
-    fo.open = 0;
-    const int r = shade<FULL, FULL, FULL>(S, cfg, ps, hit, h, id, sh, nsh, child, err, nullptr, nullptr, nullptr,
-                                          FULL ? &fo : nullptr);
+    const int r = shade<false, FULL, FULL>(S, cfg, ps, hit, h, id, sh, nsh, child, err);
     // pending: waiting branches; bit 8: the sample has split
     if (r == SHADE_SPLIT) {
       const int n = pending & 0xFF;
@@ -340,11 +335,12 @@ cudaError_t launch_megakernel(const DevScene& S, const RenderCfg& cfg, float* ou
                               unsigned long long* counters, cudaStream_t stream) {
   const uint64_t threads = (uint64_t)cfg.tiles_x * cfg.tiles_y * 32ull * (uint64_t)cfg.chunks;
   const uint32_t blocks = (uint32_t)((threads + 127) / 128);
-  // the fuller instantiation (subsurface frames, glossy lobes, parallel /
+  // the fuller instantiations (subsurface frames; glossy lobes, parallel /
   // spot / infinity lights, textures) only where needed
-  if (S.has_sss || S.has_glossy || S.n_point_lights > 0 || S.has_tex)
-    pt_megakernel<true><<<blocks, 128, 0, stream>>>(S, cfg, out, err, counters);
-  else pt_megakernel<false><<<blocks, 128, 0, stream>>>(S, cfg, out, err, counters);
+  if (S.has_sss) pt_megakernel<true, true><<<blocks, 128, 0, stream>>>(S, cfg, out, err, counters);
+  else if (S.has_glossy || S.n_point_lights > 0 || S.has_tex)
+    pt_megakernel<false, true><<<blocks, 128, 0, stream>>>(S, cfg, out, err, counters);
+  else pt_megakernel<false, false><<<blocks, 128, 0, stream>>>(S, cfg, out, err, counters);
   return cudaGetLastError();
 }
 
