@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/prender_gpu.h"
@@ -119,7 +120,8 @@ void pr_destroy(pr_ctx* c) {
                     &c->wf_neef, &c->mlt_lum, &c->mlt_path, &c->mlt_start, &c->mlt_u, &c->mlt_cur, &c->mlt_acc,
                     &c->mlt_slots})
     b->release();
-  if (c->wf_graph) cudaGraphExecDestroy(c->wf_graph);
+  for (pr::WfGraph& q : c->wf_graphs)
+    if (q.exec) cudaGraphExecDestroy(q.exec);
   if (c->batch_exec) cudaGraphExecDestroy(c->batch_exec);
   for (cudaStream_t st : c->batch_streams) cudaStreamDestroy(st);
   for (cudaEvent_t ev : c->batch_events) cudaEventDestroy(ev);
@@ -685,12 +687,24 @@ int pr::prepare_render(pr_ctx* c, const pr_camera* cam, const pr_render_params* 
 
 extern "C" {
 
-// paths in flight (slots of the wavefront pool); PR_WF_SLOTS overrides
-static unsigned int wavefront_slots() {
+// Slots of the wavefront pool (paths in flight) for a pass of n camera
+// samples; PR_WF_SLOTS overrides, a tuned size bounds it.  Every iteration's
+// launches end with their longest rays on an emptying chip, so a large frame
+// takes a large pool: mesh Cornell box 1024x768 x 64 spp, 2^21 / 2^22 / 2^23
+// slots on GB300: 281 / 269 / 268 ms.  A pass should refill it about once
+// (n / 2: paths that start together also thin out together; 3.1 M glass
+// samples 45.1 / 42.2 / 43.9 ms at 2^19 / 2^20 / 2^22, 0.96 M of the
+// subsurface scene 8.0 / 8.5 ms at 2^19 / 2^20), but below 2^19 slots the
+// launches are too small to pay for themselves: 0.48 M samples 6.8 / 5.7 /
+// 5.5 ms at 2^17 / 2^18 / all at once.
+constexpr unsigned int kWfMinSlots = 1u << 19, kWfMaxSlots = 1u << 22, kWfSpareSlots = 1u << 21;
+static unsigned int wavefront_slots(uint64_t n, unsigned int tuned) {
   const char* e = getenv("PR_WF_SLOTS");
-  long v = e ? strtol(e, nullptr, 10) : 0;
-  if (v < 1024 || v > (1L << 24)) v = 1L << 21;
-  return (unsigned int)v;
+  const long v = e ? strtol(e, nullptr, 10) : 0;
+  if (v >= 1024 && v <= (1L << 24)) return tuned ? tuned : (unsigned int)v;
+  const uint64_t want = n <= kWfMinSlots ? (n + 8191) / 8192 * 8192 : (n / 2 + 65535) / 65536 * 65536;
+  const uint64_t most = tuned ? tuned : kWfMaxSlots;
+  return (unsigned int)std::min(most, n <= kWfMinSlots ? want : std::max<uint64_t>(want, kWfMinSlots));
 }
 
 // PR_MODE_MLT (Render::RunMLT's estimator as parallel chains, mlt.cu): the
@@ -769,10 +783,37 @@ static int render_mlt(pr_ctx* c, const RenderCfg& g0, const pr_render_params* p,
   return PR_OK;
 }
 
+// The graph of a frame's loop; the context keeps the last few, since the
+// frames of a batch and previews of several sizes differ in their grids.
+// A graph that cannot be built leaves *out null: the host-driven loop runs.
+static cudaError_t wavefront_graph(pr_ctx* c, const WfLaunch& L, cudaGraphExec_t* out) {
+  *out = nullptr;
+  for (pr::WfGraph& q : c->wf_graphs)
+    if (q.exec && q.launch == L) {
+      *out = q.exec;
+      return cudaSuccess;
+    }
+  pr::WfGraph& q = c->wf_graphs[c->wf_graph_next++ % pr::kWfGraphs];
+  if (q.exec) {
+    const cudaError_t e = cudaStreamSynchronize(c->stream);  // a render that uses it has finished
+    cudaGraphExecDestroy(q.exec);
+    q.exec = nullptr;
+    if (e != cudaSuccess) return e;
+  }
+  if (wf_build_graph(L, c->stream, &q.exec) != cudaSuccess) {
+    cudaGetLastError();
+    q.exec = nullptr;
+    c->wf_graph_failed = true;
+    return cudaSuccess;
+  }
+  q.launch = L;
+  *out = q.exec;
+  return cudaSuccess;
+}
+
 static int render_wavefront(pr_ctx* c, const RenderCfg& g, float* rgb_dev, int accumulate,
                             const SceneObjData* scene = nullptr) {
   const SceneObjData& sc = scene ? *scene : c->cur;
-  const unsigned int P = c->tuned_slots ? c->tuned_slots : wavefront_slots();
   const uint64_t wh = (uint64_t)g.width * g.height;
   // camera samples per pass (sample table 28 B each); subsurface scenes take
   // smaller passes, whose frames (72 B each) come from a per-pass pool
@@ -782,36 +823,34 @@ static int render_wavefront(pr_ctx* c, const RenderCfg& g, float* rgb_dev, int a
   const uint64_t pass_cap = layers * wh;
   const uint64_t frame_cap = sss ? std::min<uint64_t>(8 * pass_cap, 1ull << 30) : 0;
   const size_t f4 = sizeof(float4);
-  PR_CUDA(c, c->wf_o.ensure(f4 * P));
-  PR_CUDA(c, c->wf_d.ensure(f4 * P));
-  PR_CUDA(c, c->wf_beta.ensure(f4 * P));
-  PR_CUDA(c, c->wf_dpw.ensure(f4 * P));
-  PR_CUDA(c, c->wf_L.ensure(f4 * P));
-  PR_CUDA(c, c->wf_sample.ensure(8ull * P));
-  PR_CUDA(c, c->wf_hit.ensure(f4 * P));
-  PR_CUDA(c, c->wf_hitv.ensure(4ull * P));
-  PR_CUDA(c, c->wf_nee.ensure(f4 * 3 * P));
-  PR_CUDA(c, c->wf_sho.ensure(f4 * 3 * P));
-  PR_CUDA(c, c->wf_shd.ensure(f4 * 3 * P));
-  PR_CUDA(c, c->wf_extq.ensure(4ull * P));
-  PR_CUDA(c, c->wf_shq.ensure(4ull * 3 * P));
-  const unsigned int spawn_cap = 2 * P;
-  PR_CUDA(c, c->wf_spo.ensure(f4 * spawn_cap));
-  PR_CUDA(c, c->wf_spd.ensure(f4 * spawn_cap));
-  PR_CUDA(c, c->wf_spb.ensure(f4 * spawn_cap));
-  PR_CUDA(c, c->wf_spw.ensure(f4 * spawn_cap));
-  PR_CUDA(c, c->wf_sps.ensure(8ull * spawn_cap));
-  PR_CUDA(c, c->wf_samp.ensure(24ull * pass_cap));
-  PR_CUDA(c, c->wf_live.ensure(4ull * pass_cap));
-  PR_CUDA(c, c->wf_pix.ensure(24ull * wh));
-  PR_CUDA(c, c->wf_ctl.ensure(sizeof(WfCtl)));
-  if (sss) {
-    PR_CUDA(c, c->wf_frc.ensure(24ull * frame_cap));
-    PR_CUDA(c, c->wf_fre.ensure(24ull * frame_cap));
-    PR_CUDA(c, c->wf_frs.ensure(f4 * frame_cap));
-    PR_CUDA(c, c->wf_frl.ensure(8ull * frame_cap));
-    PR_CUDA(c, c->wf_spf.ensure(4ull * spawn_cap));
-    PR_CUDA(c, c->wf_neef.ensure(4ull * P));
+  // the pool; where the device cannot hold a large one, a smaller one
+  unsigned int P = wavefront_slots(pass_cap, c->tuned_slots), spawn_cap = 0;
+  for (;;) {
+    // glass branches that wait: more of them than slots where a frame's paths
+    // all start at once
+    spawn_cap = 2 * std::max(P, kWfSpareSlots);
+    const std::pair<DevBuf*, size_t> pool[] = {
+        {&c->wf_o, f4 * P}, {&c->wf_d, f4 * P}, {&c->wf_beta, f4 * P}, {&c->wf_dpw, f4 * P}, {&c->wf_L, f4 * P},
+        {&c->wf_sample, 8ull * P}, {&c->wf_hit, f4 * P}, {&c->wf_hitv, 4ull * P}, {&c->wf_nee, f4 * 3 * P},
+        {&c->wf_sho, f4 * 3 * P}, {&c->wf_shd, f4 * 3 * P}, {&c->wf_extq, 4ull * P}, {&c->wf_shq, 4ull * 3 * P},
+        {&c->wf_spo, f4 * spawn_cap}, {&c->wf_spd, f4 * spawn_cap}, {&c->wf_spb, f4 * spawn_cap},
+        {&c->wf_spw, f4 * spawn_cap}, {&c->wf_sps, 8ull * spawn_cap}, {&c->wf_samp, 24ull * pass_cap},
+        {&c->wf_live, 4ull * pass_cap}, {&c->wf_pix, 24ull * wh}, {&c->wf_ctl, sizeof(WfCtl)},
+        {sss ? &c->wf_frc : nullptr, 24ull * frame_cap}, {sss ? &c->wf_fre : nullptr, 24ull * frame_cap},
+        {sss ? &c->wf_frs : nullptr, f4 * frame_cap}, {sss ? &c->wf_frl : nullptr, 8ull * frame_cap},
+        {sss ? &c->wf_spf : nullptr, 4ull * spawn_cap}, {sss ? &c->wf_neef : nullptr, 4ull * P}};
+    cudaError_t e = cudaSuccess;
+    for (const auto& q : pool)
+      if (q.first && e == cudaSuccess) e = q.first->ensure(q.second);
+    if (e == cudaErrorMemoryAllocation && P > kWfSpareSlots && !c->tuned_slots && !getenv("PR_WF_SLOTS")) {
+      cudaGetLastError();
+      P = kWfSpareSlots;
+      for (const auto& q : pool)
+        if (q.first) q.first->release();
+      continue;
+    }
+    PR_CUDA(c, e);
+    break;
   }
   if (!c->wf_host_ctl) PR_CUDA(c, cudaMallocHost((void**)&c->wf_host_ctl, sizeof(WfCtl)));
   WfBufs B{};
@@ -850,7 +889,6 @@ static int render_wavefront(pr_ctx* c, const RenderCfg& g, float* rgb_dev, int a
   B.spawn_cap = spawn_cap;
   B.max_iterations = 20000u;  // bounded device loop; a frame needs a few hundred
   WfLaunch L;
-  L.shade_blocks = (P + 127) / 128;
   L.sss = sss ? 1 : 0;
   L.ext = (sc.dev.n_point_lights > 0 || sc.dev.has_tex) ? 1 : 0;
   // persistent traversal: one resident wave of blocks (more waves only queue
@@ -858,7 +896,8 @@ static int render_wavefront(pr_ctx* c, const RenderCfg& g, float* rgb_dev, int a
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess || sms <= 0) sms = 152;
   const unsigned int bps = c->tuned_trace_bps ? c->tuned_trace_bps : kTraceBlocksPerSM;
-  L.trace_blocks = std::min<unsigned int>((P + 127) / 128, (unsigned int)sms * bps);
+  L.trace_blocks = (unsigned int)sms * bps;
+  L.shade_blocks = (P + 127) / 128;
   PR_CUDA(c, cudaMemsetAsync(c->wf_nee.p, 0, f4 * 3 * P, c->stream));
   PR_CUDA(c, cudaMemsetAsync(B.pix, 0, 24ull * wh, c->stream));
   if (sss) {
@@ -870,25 +909,8 @@ static int render_wavefront(pr_ctx* c, const RenderCfg& g, float* rgb_dev, int a
   // conditional graph nodes see every launch this way (same kernels, same work)
   const char* host_loop = getenv("PR_WF_HOST_LOOP");
   const bool use_graph = !(host_loop && host_loop[0] == '1') && !c->force_host_loop;
-  if (use_graph && !c->wf_graph_failed &&
-      (!c->wf_graph || c->wf_graph_slots != P || c->wf_graph_trace_blocks != L.trace_blocks ||
-       c->wf_graph_variant != L.sss + 2 * L.ext)) {
-    if (c->wf_graph) {
-      cudaStreamSynchronize(c->stream);  // the previous render's launch has finished with it
-      cudaGraphExecDestroy(c->wf_graph);
-    }
-    c->wf_graph = nullptr;
-    cudaError_t e = wf_build_graph(L, c->stream, &c->wf_graph);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      c->wf_graph = nullptr;
-      c->wf_graph_failed = true;  // fall back to the host-driven loop
-    } else {
-      c->wf_graph_slots = P;
-      c->wf_graph_trace_blocks = L.trace_blocks;
-      c->wf_graph_variant = L.sss + 2 * L.ext;
-    }
-  }
+  cudaGraphExec_t graph = nullptr;
+  if (use_graph && !c->wf_graph_failed) PR_CUDA(c, wavefront_graph(c, L, &graph));
   c->wf_passes = 0;
   for (double& t : c->kernel_ms) t = 0.0;
   for (uint64_t first = 0; first < (uint64_t)g.spp; first += layers) {
@@ -899,7 +921,7 @@ static int render_wavefront(pr_ctx* c, const RenderCfg& g, float* rgb_dev, int a
     PR_CUDA(c, cudaMemsetAsync(B.samp, 0, 24ull * B.pass_samples, c->stream));
     PR_CUDA(c, wf_set_constants(sc.dev, g, B, c->stream));
     PR_CUDA(c, wf_reset_launch(P, c->stream));
-    if (use_graph && c->wf_graph) PR_CUDA(c, cudaGraphLaunch(c->wf_graph, c->stream));
+    if (graph) PR_CUDA(c, cudaGraphLaunch(graph, c->stream));
     else PR_CUDA(c, wf_run_host_loop(L, c->wf_host_ctl, (const WfCtl*)B.ctl, c->stream, c->kernel_ms));
   }
   PR_CUDA(c, wf_resolve_launch(rgb_dev, (int)(3 * wh), accumulate, g.sensor, c->stream));

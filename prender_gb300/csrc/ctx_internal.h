@@ -32,6 +32,13 @@ struct DevBuf {
   }
 };
 
+// a wavefront graph and the launches in it
+constexpr int kWfGraphs = 8;
+struct WfGraph {
+  WfLaunch launch{};
+  cudaGraphExec_t exec = nullptr;
+};
+
 // one uploaded scene: host build, device copies, device view
 struct SceneObjData {
   HostScene host;
@@ -75,10 +82,8 @@ struct pr_ctx {
   pr::DevBuf wf_spo, wf_spd, wf_spb, wf_spw, wf_sps, wf_samp, wf_live, wf_pix, wf_ctl;
   pr::DevBuf wf_frc, wf_fre, wf_frs, wf_frl, wf_spf, wf_neef;  // subsurface frames (wavefront form)
   unsigned int wf_slots = 0;
-  cudaGraphExec_t wf_graph = nullptr;
-  unsigned int wf_graph_slots = 0;
-  unsigned int wf_graph_trace_blocks = 0;
-  int wf_graph_variant = 0;          // shading kernel the graph launches: sss + 2 * ext
+  pr::WfGraph wf_graphs[pr::kWfGraphs];
+  unsigned int wf_graph_next = 0;    // the entry that the next new graph takes
   unsigned int tuned_slots = 0;      // autotuner's wavefront pool size (0: default)
   unsigned int tuned_trace_bps = 0;  // autotuner's traversal blocks per SM (0: default)
   bool force_host_loop = false;      // the autotuner times candidates with the host-driven loop

@@ -73,6 +73,9 @@ struct WfLaunch {
   unsigned int trace_blocks;
   int sss;    // the scene has subsurface materials: the fuller shading kernel with frames
   int ext;    // the scene has parallel, spot or infinity lights, textures or IBL images
+  bool operator==(const WfLaunch& o) const {
+    return shade_blocks == o.shade_blocks && trace_blocks == o.trace_blocks && sss == o.sss && ext == o.ext;
+  }
 };
 
 cudaError_t wf_set_constants(const DevScene& S, const RenderCfg& cfg, const WfBufs& B, cudaStream_t s);
