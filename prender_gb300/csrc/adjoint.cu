@@ -325,7 +325,7 @@ cudaError_t launch_adjoint(const DevScene& S, const RenderCfg& cfg, const float*
       A.item = reinterpret_cast<unsigned long long*>(A.ew + 3 * n);
       A.anc = reinterpret_cast<int*>(A.item + n);
       A.carry = reinterpret_cast<float*>(p + (h.slot_bytes * n + 255) / 256 * 256);
-      adjoint_paths<<<b.blocks, b.threads, block_shared_bytes(b.slots), stream>>>(S, cfg, A, P, dl_drgb, err, counters);
+      adjoint_paths<<<b.blocks, b.threads, block_shared_bytes(b), stream>>>(S, cfg, A, P, dl_drgb, err, counters);
       e = cudaGetLastError();
       if (e != cudaSuccess) return e;
       adjoint_reduce<<<(warps + 3) / 4, 128, 0, stream>>>(A, d_color, d_emission);

@@ -106,13 +106,16 @@ __device__ __forceinline__ int block_pop(const BlockPool& P, size_t i, int n, Pa
 // The trace phase: rays [0, n_ext) of extq, then [n_ext, n_ext + n_sh) of shq.
 __device__ __forceinline__ void block_trace(const DevScene& S, const BlockPool& P, size_t base, BlockShared& B,
                                             const unsigned short* extq, const unsigned short* shq,
-                                            unsigned char* lit, TraceStats& st, uint32_t& segs, uint32_t* err) {
+                                            unsigned char* lit, float4* found, TraceStats& st, uint32_t& segs,
+                                            uint32_t* err) {
   const int lane = threadIdx.x & 31;
   const unsigned int n_ext = B.n_ext, n = n_ext + B.n_sh;
   const unsigned int warps = blockDim.x / 32;
   // few rays spread over all warps
   const int width = (int)min(32u, (n + warps - 1) / warps);
   TraceLane r;
+  lane_start(r, f3(0, 0, 0), f3(0, 0, 1), 0.0f);
+  r.any = false;
   WGroup stack[kWStack];
   int item = 0;
   bool busy = false, exhausted = lane >= width;
@@ -151,7 +154,7 @@ __device__ __forceinline__ void block_trace(const DevScene& S, const BlockPool& 
         }
       }
     }
-    if (busy && trace_step<TRACE_EITHER>(S, r, stack, st, err)) {
+    if (trace_step<TRACE_EITHER>(S, busy, r, stack, found, st, err)) {
       busy = false;
       if (r.any) {
         lit[item] = r.h.ent < 0;
@@ -175,7 +178,8 @@ template <class D>
 __device__ __forceinline__ void block_paths(const DevScene& S, const BlockPool& P, D& drv, unsigned char* smem,
                                             TraceStats& st, uint32_t& segs, uint32_t* err) {
   BlockShared& B = *reinterpret_cast<BlockShared*>(smem);
-  unsigned short* extq = reinterpret_cast<unsigned short*>(smem + sizeof(BlockShared));
+  float4* found = reinterpret_cast<float4*>(smem + sizeof(BlockShared)) + (threadIdx.x & ~31u);  // warp_triangles
+  unsigned short* extq = reinterpret_cast<unsigned short*>(smem + sizeof(BlockShared) + 16 * blockDim.x);
   unsigned short* shq = extq + P.slots;
   unsigned char* lit = reinterpret_cast<unsigned char*>(shq + 3 * P.slots);
   unsigned char* alive = lit + 4 * P.slots;
@@ -249,7 +253,7 @@ __device__ __forceinline__ void block_paths(const DevScene& S, const BlockPool& 
       if (tid == 0) atomicOr(err, PR_DEV_LOOP_CAP);
       break;
     }
-    block_trace(S, P, base, B, extq, shq, lit, st, segs, err);
+    block_trace(S, P, base, B, extq, shq, lit, found, st, segs, err);
   }
 }
 
@@ -319,6 +323,8 @@ inline BlockPool block_pool(void* p, size_t n) {
 }
 
 // dynamic shared memory of block_paths
-inline size_t block_shared_bytes(int slots) { return sizeof(BlockShared) + (2 + 6 + 4 + 1) * (size_t)slots; }
+inline size_t block_shared_bytes(const BlockShape& b) {
+  return sizeof(BlockShared) + 16 * (size_t)b.threads + (2 + 6 + 4 + 1) * (size_t)b.slots;
+}
 
 }  // namespace pr

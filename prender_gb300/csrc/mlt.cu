@@ -358,7 +358,7 @@ cudaError_t run_paths(const DevScene& S, const RenderCfg& cfg, MltRun R, unsigne
   R.it = reinterpret_cast<int64_t*>(p);
   R.chain = reinterpret_cast<int*>(R.it + slots);
   R.pix = R.chain + slots;
-  mlt_paths<SEEDS><<<b.blocks, b.threads, block_shared_bytes(b.slots), stream>>>(S, cfg, R, P, err, counters);
+  mlt_paths<SEEDS><<<b.blocks, b.threads, block_shared_bytes(b), stream>>>(S, cfg, R, P, err, counters);
   return cudaGetLastError();
 }
 

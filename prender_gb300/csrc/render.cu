@@ -321,7 +321,7 @@ cudaError_t launch_plain(const DevScene& S, const RenderCfg& cfg, void* scratch,
   BlockPool P = block_pool(static_cast<char*>(scratch) + pixel_bytes(cfg), (size_t)b.blocks * b.slots);
   P.slots = b.slots;
   P.slots_used = b.used;
-  const size_t smem = block_shared_bytes(b.slots);
+  const size_t smem = block_shared_bytes(b);
   if (S.has_glossy || S.n_point_lights > 0 || S.has_tex)
     pt_block<true><<<b.blocks, b.threads, smem, stream>>>(S, cfg, F, P, err, counters);
   else

@@ -507,17 +507,15 @@ __device__ __forceinline__ bool mesh_bounds_hit(const GEntF& e, const WRay& r, f
   return tn <= tf;
 }
 
-// One step of a ray: the other entities up to the next mesh the ray may meet
-// (if it is not in one), then one node of that mesh with its leaf triangles
-// (fast_qbvh's loop body), so that a lane that starts a ray or a mesh shares
-// the warp's node visit.  True when the ray is answered (any hit: h.ent >= 0
-// means occluded).  Measured and not kept, within 2 % on GB300: voting per
-// step between entity, node and triangle work (16 to 20 lanes a step instead
-// of 11, paid back in votes), two triangles side by side, the next node's
-// prefetch (3 % slower).
+// One step of a ray, in three parts: trace_visit goes through the other
+// entities up to the next mesh the ray may meet (if it is not in one) and
+// visits one node of that mesh; warp_triangles tests the triangles of the
+// leaves that the warp's rays hit there; trace_next leaves a finished mesh.
+// True when the ray is answered (any hit: h.ent >= 0 means occluded).
+// tm, tb: the node's triangles to test (bit k: triangle slot tb + k).
 template <int MODE>
-__device__ __forceinline__ bool trace_step(const DevScene& S, TraceLane& r, WGroup* stack, TraceStats& st,
-                                           uint32_t* err) {
+__device__ __forceinline__ bool trace_visit(const DevScene& S, TraceLane& r, WGroup* stack, TraceStats& st,
+                                            uint32_t* err, uint32_t& tm, int& tb) {
   const bool any = MODE == TRACE_ANY || (MODE == TRACE_EITHER && r.any);
   if (!r.in_mesh) {
     while (r.ent < S.n_ents) {
@@ -572,30 +570,102 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, TraceLane& r, WGro
     stack[r.sp++] = r.g;
   }
   st.nodes++;
-  uint32_t tm;
-  int tb;
   wnode_visit(S.rnodes + child, r.ray, r.tmax, r.g, tm, tb);
-  while (tm) {
-    const int k = __ffs(tm) - 1;
-    tm &= tm - 1u;
-    st.tris++;
-    float t, uu, vv;
-    if (fast_tri(S.rtris + 3 * (size_t)(tb + k), r.ray.o, r.ray.d, r.tmax, t, uu, vv)) {
-      r.h.ent = r.ent;
-      r.h.slot = tb + k;
-      if (any) return true;
-      r.tmax = t;
-      r.h.t = t;
-      r.h.u = uu;
-      r.h.v = vv;
-    }
+  return false;
+}
+
+// The triangles of a step (tm, tb of every lane; none where tm is 0), spread
+// over the warp: a node visit leaves 1.25 triangles a ray on average but many
+// on some, and tested by their own lanes they were more than half of the
+// traversal's instructions at some six lanes each.  Lane j takes the j-th
+// (ray, triangle) pair, its ray by shuffles; a hit goes to the warp's 32
+// entries of `found`, and the ray's lane takes its hits in the order of its
+// triangles, the strictly closest first, as one lane alone would.
+// True where an any-hit ray met a triangle.  All lanes of the warp.
+template <int MODE>
+__device__ __forceinline__ bool warp_triangles(const DevScene& S, TraceLane& r, uint32_t tm, int tb, float4* found,
+                                               TraceStats& st) {
+  if (!__any_sync(0xffffffffu, tm != 0)) return false;
+  const bool any = MODE == TRACE_ANY || (MODE == TRACE_EITHER && r.any);
+  const int lane = threadIdx.x & 31, cnt = __popc(tm);
+  int incl = cnt;  // pairs of lanes 0..lane
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += v;
   }
+  const int total = __shfl_sync(0xffffffffu, incl, 31), excl = incl - cnt;
+  bool met = false;
+  for (int base = 0; base < total; base += 32) {
+    const int j = base + lane;
+    int own = 0;  // the lane of pair j: the number of lanes with incl <= j
+#pragma unroll
+    for (int s = 16; s; s >>= 1)
+      if (__shfl_sync(0xffffffffu, incl, own + s - 1) <= j) own += s;
+    int k = j - __shfl_sync(0xffffffffu, excl, own);
+    uint32_t m = __shfl_sync(0xffffffffu, tm, own);
+    int slot = __shfl_sync(0xffffffffu, tb, own);
+    const float3 o = f3(__shfl_sync(0xffffffffu, r.ray.o.x, own), __shfl_sync(0xffffffffu, r.ray.o.y, own),
+                        __shfl_sync(0xffffffffu, r.ray.o.z, own));
+    const float3 d = f3(__shfl_sync(0xffffffffu, r.ray.d.x, own), __shfl_sync(0xffffffffu, r.ray.d.y, own),
+                        __shfl_sync(0xffffffffu, r.ray.d.z, own));
+    const float tmax = __shfl_sync(0xffffffffu, r.tmax, own);
+    bool hit = false;
+    if (j < total) {
+      for (; k > 0; k--) m &= m - 1u;
+      slot += __ffs(m) - 1;
+      float t, u, v;
+      hit = fast_tri(S.rtris + 3 * (size_t)slot, o, d, tmax, t, u, v);
+      if (hit) found[lane] = make_float4(t, u, v, __int_as_float(slot));
+    }
+    const uint32_t hits = __ballot_sync(0xffffffffu, hit);  // orders found[] too
+    const int lo = max(excl - base, 0), hi = min(incl - base, 32);
+    if (hits && hi > lo && !met) {
+      uint32_t mine = hits & (0xffffffffu >> (32 - (hi - lo))) << lo;
+      while (mine) {
+        const int q = __ffs(mine) - 1;
+        mine &= mine - 1u;
+        const float4 f = found[q];
+        if (!(f.x < r.tmax)) continue;
+        r.h.ent = r.ent;
+        r.h.slot = __float_as_int(f.w);
+        if (any) {
+          met = true;
+          st.tris += base + q - excl + 1;
+          break;
+        }
+        r.tmax = f.x;
+        r.h.t = f.x;
+        r.h.u = f.y;
+        r.h.v = f.z;
+      }
+    }
+    __syncwarp();
+  }
+  if (!met) st.tris += cnt;
+  return met;
+}
+
+// leaves a mesh whose nodes are all visited; true past the last entity
+__device__ __forceinline__ bool trace_next(const DevScene& S, TraceLane& r) {
   if ((r.g.bits & 0xFFu) == 0 && r.sp == 0) {
     r.in_mesh = false;  // this mesh is done
     r.ent++;
     return r.ent >= S.n_ents;
   }
   return false;
+}
+
+// One step of all lanes of a warp; true for a lane whose ray is answered.
+template <int MODE>
+__device__ __forceinline__ bool trace_step(const DevScene& S, bool busy, TraceLane& r, WGroup* stack, float4* found,
+                                           TraceStats& st, uint32_t* err) {
+  uint32_t tm = 0;
+  int tb = 0;
+  bool done = busy && trace_visit<MODE>(S, r, stack, st, err, tm, tb);
+  const bool met = warp_triangles<MODE>(S, r, tm, tb, found, st);
+  if (busy && !done) done = met || trace_next(S, r);
+  return done;
 }
 
 // closest hit over the entity list (strict '<' in list order)

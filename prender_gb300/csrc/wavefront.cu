@@ -443,7 +443,9 @@ __device__ __forceinline__ void persistent_trace(const DevScene& S, unsigned int
   // few rays spread over all warps
   const unsigned int warps = gridDim.x * (blockDim.x / 32);
   const int width = (int)min(32u, (n + warps - 1) / warps);
+  __shared__ float4 found[128];
   TraceLane r;
+  lane_start(r, f3(0, 0, 0), f3(0, 0, 1), 0.0f);
   WGroup stack[kWStack];
   bool busy = false, exhausted = lane >= width;
   for (unsigned int step = 0;; step++) {
@@ -470,7 +472,7 @@ __device__ __forceinline__ void persistent_trace(const DevScene& S, unsigned int
         }
       }
     }
-    if (busy && trace_step<ANY ? TRACE_ANY : TRACE_CLOSEST>(S, r, stack, st, err)) {
+    if (trace_step<ANY ? TRACE_ANY : TRACE_CLOSEST>(S, busy, r, stack, found + (threadIdx.x & ~31u), st, err)) {
       finish(r);
       busy = false;
     }
