@@ -677,7 +677,7 @@ int pr::prepare_render(pr_ctx* c, const pr_camera* cam, const pr_render_params* 
   g.sample_offset = sample_offset;
   g.tiles_x = (uint32_t)((cam->width + 7) / 8);
   g.tiles_y = (uint32_t)((cam->height + 3) / 4);
-  // enough sample chunks to keep ~1.2M threads in flight
+  // enough sample chunks to keep ~1.2M threads in flight (pt_megakernel, the adjoint's sums)
   const double pixels = (double)cam->width * cam->height;
   int chunks = (int)std::ceil(1.2e6 / pixels);
   chunks = std::max(1, std::min(chunks, g.spp));
@@ -693,17 +693,18 @@ extern "C" {
 // takes a large pool: mesh Cornell box 1024x768 x 64 spp, 2^21 / 2^22 / 2^23
 // slots on GB300: 281 / 269 / 268 ms.  A pass should refill it about once
 // (n / 2: paths that start together also thin out together; 3.1 M glass
-// samples 45.1 / 42.2 / 43.9 ms at 2^19 / 2^20 / 2^22, 0.96 M of the
-// subsurface scene 8.0 / 8.5 ms at 2^19 / 2^20), but below 2^19 slots the
+// samples 45.1 / 42.2 / 43.9 ms at 2^19 / 2^20 / 2^22), or in subsurface
+// scenes, whose paths are longer, a few times (n / 4: 4 M of their samples
+// 38 / 37 / 40 ms at 2^19 / 2^20 / 2^21), but below 2^19 slots the
 // launches are too small to pay for themselves: 0.48 M samples 6.8 / 5.7 /
 // 5.5 ms at 2^17 / 2^18 / all at once.
 constexpr unsigned int kWfMinSlots = 1u << 19, kWfMaxSlots = 1u << 22, kWfSpareSlots = 1u << 21;
-static unsigned int wavefront_slots(uint64_t n, unsigned int tuned) {
+static unsigned int wavefront_slots(uint64_t n, unsigned int tuned, bool sss) {
   const char* e = getenv("PR_WF_SLOTS");
   const long v = e ? strtol(e, nullptr, 10) : 0;
   if (v >= 1024 && v <= (1L << 24)) return tuned ? tuned : (unsigned int)v;
-  const uint64_t want = n <= kWfMinSlots ? (n + 8191) / 8192 * 8192 : (n / 2 + 65535) / 65536 * 65536;
-  const uint64_t most = tuned ? tuned : kWfMaxSlots;
+  const uint64_t want = n <= kWfMinSlots ? (n + 8191) / 8192 * 8192 : (n / (sss ? 4 : 2) + 65535) / 65536 * 65536;
+  const uint64_t most = tuned ? tuned : sss ? kWfSpareSlots : kWfMaxSlots;
   return (unsigned int)std::min(most, n <= kWfMinSlots ? want : std::max<uint64_t>(want, kWfMinSlots));
 }
 
@@ -815,17 +816,23 @@ static int render_wavefront(pr_ctx* c, const RenderCfg& g, float* rgb_dev, int a
                             const SceneObjData* scene = nullptr) {
   const SceneObjData& sc = scene ? *scene : c->cur;
   const uint64_t wh = (uint64_t)g.width * g.height;
-  // camera samples per pass (sample table 28 B each); subsurface scenes take
-  // smaller passes, whose frames (72 B each) come from a per-pass pool
   const bool sss = sc.dev.has_sss != 0;
-  const uint64_t max_pass = sss ? (4ull << 20) : (64ull << 20);
-  uint64_t layers = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)g.spp, max_pass / wh));
-  const uint64_t pass_cap = layers * wh;
-  const uint64_t frame_cap = sss ? std::min<uint64_t>(8 * pass_cap, 1ull << 30) : 0;
   const size_t f4 = sizeof(float4);
-  // the pool; where the device cannot hold a large one, a smaller one
-  unsigned int P = wavefront_slots(pass_cap, c->tuned_slots), spawn_cap = 0;
-  for (;;) {
+  // the pool, and the camera samples of a pass (sample table 28 B each).
+  // Subsurface scenes take smaller passes, whose frames (8 a sample, 72 B
+  // each) come from a per-pass pool: every pass ends with its longest paths,
+  // 64 spp at 1024x1024 in passes of 4 / 8 / 16 / 32 M samples 594 / 549 /
+  // 518 / 499 ms, the frames of 16 M being 9.7 GB.  Where the device cannot
+  // hold that, a smaller pool and passes of 4 M.
+  uint64_t layers = 0, pass_cap = 0, frame_cap = 0;
+  unsigned int P = 0, spawn_cap = 0;
+  for (bool less = false;; less = true) {
+    const uint64_t max_pass = !sss ? (64ull << 20) : less ? (4ull << 20) : (16ull << 20);
+    layers = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)g.spp, max_pass / wh));
+    pass_cap = layers * wh;
+    frame_cap = sss ? std::min<uint64_t>(8 * pass_cap, 1ull << 30) : 0;
+    P = wavefront_slots(pass_cap, c->tuned_slots, sss);
+    if (less && !c->tuned_slots && !getenv("PR_WF_SLOTS")) P = std::min(P, kWfSpareSlots);
     // glass branches that wait: more of them than slots where a frame's paths
     // all start at once
     spawn_cap = 2 * std::max(P, kWfSpareSlots);
@@ -842,9 +849,8 @@ static int render_wavefront(pr_ctx* c, const RenderCfg& g, float* rgb_dev, int a
     cudaError_t e = cudaSuccess;
     for (const auto& q : pool)
       if (q.first && e == cudaSuccess) e = q.first->ensure(q.second);
-    if (e == cudaErrorMemoryAllocation && P > kWfSpareSlots && !c->tuned_slots && !getenv("PR_WF_SLOTS")) {
+    if (e == cudaErrorMemoryAllocation && !less) {
       cudaGetLastError();
-      P = kWfSpareSlots;
       for (const auto& q : pool)
         if (q.first) q.first->release();
       continue;
@@ -983,7 +989,7 @@ int pr_render_dev(pr_ctx* c, const pr_camera* cam, const pr_render_params* p, fl
   const bool mlt = p->mode == PR_MODE_MLT && !kerr && !worm;
   // MLT: paths = bootstrap paths + proposals
   const uint64_t paths = wf ? (uint64_t)g.spp * g.width * g.height : mlt ? mlt_paths : cnt[0];
-  // wavefront: reset per pass + 4 per iteration + resolve; megakernel: kernel + reduce;
+  // wavefront: reset per pass + 4 per iteration + resolve; plain: kernel + resolve or reduce;
   // MLT: bootstrap, chain start, the chains' launches, resolve
   const uint64_t launches = wf ? 4 * cnt[5] + c->wf_passes + 1 : mlt ? mlt_launches : kerr ? (uint64_t)kerr_render_launches(c->cur.kerr) : 2;
   // Kerr counters: [1] accepted RK steps, [2] RK attempts, [3] segment scene
@@ -1448,13 +1454,12 @@ int pr_kerr_sensitivity_adjoint(pr_ctx* c, const double* rays, int64_t n, const 
   return kerr_sens_common(c, rays, n, basis, cotangent, nullptr, nullptr, nullptr, grad);
 }
 
-// the plain form of this scene is the stream kernel (straight rays, no subsurface materials)
-static bool streamed(const SceneObjData& sc) { return !sc.kerr.enabled && !sc.worm.enabled && !sc.dev.has_sss; }
+// the plain form of this scene is the block kernel (straight rays, no subsurface materials)
+static bool block_form(const SceneObjData& sc) { return !sc.kerr.enabled && !sc.worm.enabled && !sc.dev.has_sss; }
 
 // Many jobs (scene object, camera, parameters, output) as one captured CUDA
-// graph: each job is the megakernel form (one render kernel + the ordered
-// chunk reduction) on its own branch of the graph, so small and large
-// frames overlap on the GPU; the graph is re-captured per call and updated
+// graph: each job is the plain form (or a Kerr or wormhole frame) on its own
+// branch of the graph, so small and large frames overlap on the GPU; the graph is re-captured per call and updated
 // in place when its shape is unchanged.
 int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
   if (!c) return PR_E_ARG;
@@ -1477,7 +1482,7 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
       return fail(c, PR_E_UNSUPPORTED, "job " + std::to_string(j) + ": Metropolis renders run through pr_render");
     int st = prepare_render(c, &J.camera, &J.params, J.sample_offset, cfg[j], &J.scene->data);
     if (st != PR_OK) return fail(c, st, "job " + std::to_string(j) + ": " + c->err);
-    // the batch fills the GPU with many jobs: fewer sample chunks per job
+    // the batch fills the GPU with many jobs: fewer sample chunks per job (subsurface scenes)
     cfg[j].chunks = std::max(1, std::min(cfg[j].chunks, (int)std::ceil(2.0e5 / ((double)cfg[j].width * cfg[j].height))));
     cfg[j].chunks = std::min(cfg[j].chunks, cfg[j].spp);
     const SceneObjData& sc = J.scene->data;
@@ -1485,7 +1490,7 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
     if (J.params.mode == PR_MODE_WAVEFRONT && !sc.kerr.enabled && !sc.worm.enabled) bytes = 0;
     else if (sc.kerr.enabled) bytes = kerr_scratch_bytes(sc.kerr, cfg[j]);
     else if (sc.worm.enabled) bytes = worm_scratch_bytes(cfg[j]);
-    else if (streamed(sc)) bytes = plain_scratch_bytes(cfg[j]);
+    else if (block_form(sc)) bytes = plain_scratch_bytes(cfg[j]);
     size_t& room = branch_room[j % n_streams];
     room = std::max(room, (bytes + 255) / 256 * 256);
     paths += (uint64_t)cfg[j].spp * cfg[j].width * cfg[j].height;
@@ -1510,7 +1515,7 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
   }
   PR_CUDA(c, cudaMemsetAsync(c->errword.p, 0, 4, c->stream));
   PR_CUDA(c, cudaMemsetAsync(c->counters.p, 0, 128, c->stream));
-  // capture: fork to the branch streams, one megakernel + reduce per job, join
+  // capture: fork to the branch streams, each job's launches, join
   cudaGraph_t graph = nullptr;
   PR_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t e = cudaEventRecord(c->batch_events[n_streams], c->stream);
@@ -1524,7 +1529,7 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
     const SceneObjData& sc = J.scene->data;
     const int n3 = cfg[j].width * cfg[j].height * 3;
     float* partial = (float*)(part + off[j % n_streams]);
-    if (streamed(sc)) {
+    if (block_form(sc)) {
       e = launch_plain(sc.dev, cfg[j], partial, J.rgb_dev, J.accumulate, (uint32_t*)c->errword.p,
                         (unsigned long long*)c->counters.p, st);
       continue;

@@ -1,4 +1,4 @@
-// Wavefront renderer: the same estimator as the megakernel (path_logic.cuh),
+// Wavefront renderer: the same estimator as the plain form (path_logic.cuh),
 // scheduled as a loop of small kernels over a pool of P path slots held in
 // HBM as structure-of-arrays:
 //
@@ -417,9 +417,9 @@ __global__ void __launch_bounds__(128, 6) wf_shade() { wf_shade_impl<false, fals
 // scenes with parallel, spot or infinity lights, textures or IBL images
 __global__ void __launch_bounds__(128, 4) wf_shade_ext() { wf_shade_impl<false, true>(); }
 // scenes with subsurface materials (any light kind)
-// (96 registers: 3 / 4 / 5 blocks took 14.8 / 13.9 / 13.3 ms of a 320x320 x
-// 16 spp media frame with a 20,480-triangle subsurface mesh)
-__global__ void __launch_bounds__(128, 5) wf_shade_sss() { wf_shade_impl<true, true>(); }
+// (128 registers; a 1024x1024 x 64 spp media frame with a 20,480-triangle
+// subsurface mesh with 4 / 5 / 6 blocks: 600 / 609 ms and 3 % more)
+__global__ void __launch_bounds__(128, 4) wf_shade_sss() { wf_shade_impl<true, true>(); }
 
 // Persistent traversal with ray replacement (Aila & Laine 2009, "Understanding
 // the efficiency of ray traversal on GPUs", dynamic ray fetch): the lanes of a
