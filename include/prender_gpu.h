@@ -461,7 +461,7 @@ int pr_render(pr_ctx* ctx, const pr_camera* cam, const pr_render_params* prm,
 int pr_render_dev(pr_ctx* ctx, const pr_camera* cam, const pr_render_params* prm,
                   float* rgb_accum_dev, uint64_t sample_offset, int accumulate);
 
-/* Allocation-free variant of pr_render_dev for the megakernel form (no
+/* Allocation-free variant of pr_render_dev for the plain form (no
  * counterpart in the reference, which renders on the CPU).  For callers that
  * must not allocate device memory while rendering: a frame loop with a hard
  * time budget, which cannot absorb the device-wide synchronisation that
@@ -476,11 +476,11 @@ int pr_render_dev(pr_ctx* ctx, const pr_camera* cam, const pr_render_params* prm
  * any stream capture starts.  The kept address is not valid in a context
  * made with the driver API, nor after cudaDeviceReset.  Calls that overlap
  * on the GPU share the array and race.  The scene must already be uploaded
- * with pr_scene_upload (which allocates, at set-up).  Result as
- * pr_render_dev, except where pr_render_dev's per-chunk partial images
- * (min(ceil(1.2e6 / pixels), spp) chunks of W*H*3 floats) would not fit in
- * the array: there the samples are summed in fewer chunks, so the image
- * agrees with pr_render_dev's to float rounding rather than bit for bit. */
+ * with pr_scene_upload (which allocates, at set-up).  It traces the paths of
+ * pr_render_dev, one thread per pixel and sample chunk; the image agrees with
+ * pr_render_dev's to float rounding (pr_render_dev adds samples in fixed
+ * point, this call in min(ceil(1.2e6 / pixels), spp) float chunks, or in
+ * fewer where their partial images would not fit in the array). */
 int pr_render_dev_noalloc(pr_ctx* ctx, const pr_camera* cam, const pr_render_params* prm, float* rgb_accum_dev,
                           uint64_t sample_offset, int accumulate);
 
@@ -524,7 +524,7 @@ void pr_scene_release(pr_ctx* ctx, pr_scene_obj* scene);
 typedef struct pr_job {
   const pr_scene_obj* scene;
   pr_camera camera;
-  pr_render_params params;    /* params.mode: plain (megakernel) or wavefront form */
+  pr_render_params params;    /* params.mode: plain or wavefront form             */
   float* rgb_dev;             /* W*H*3 floats on the device, image row order  */
   uint64_t sample_offset;
   int32_t accumulate;
@@ -534,8 +534,8 @@ typedef struct pr_job {
 /* Renders n jobs (no reference counterpart: the reference renders one scene
  * per process).  Plain-form jobs (and Kerr scenes) run as one captured CUDA
  * graph, on parallel branches; each such image equals pr_render_dev of the
- * same inputs up to float summation order (a batch uses fewer sample chunks
- * per pixel).  Wavefront-form jobs share the context's path pool and run one
+ * same inputs, in subsurface scenes up to float summation order (a batch uses
+ * fewer sample chunks per pixel there).  Wavefront-form jobs share the context's path pool and run one
  * after another after that graph, each as pr_render_dev would run it (one
  * graph launch per pass), with the same image.  Scene objects must stay
  * alive until the call returns. */

@@ -1,13 +1,18 @@
-// Plain drop-in renderer (megakernel): one thread per (pixel, sample chunk)
-// runs Render::Run's per-sample body (render.h:1203-1385) -- camera ray,
-// the whole radiance() branch tree, luminance clamp -- with the per-vertex
-// logic of path_logic.cuh.  Shadow rays and the next segment are traced in
-// place; the refracted branch of a depth <= 2 glass split waits on a
-// 4-entry stack (at most three splits are pending at once: depths 0, 1, 2).
+// Plain drop-in renderer: Render::Run's per-sample body (render.h:1203-1385)
+// -- camera ray, the whole radiance() branch tree, luminance clamp -- with
+// the per-vertex logic of path_logic.cuh, in one kernel and in two shapes:
 //
-// Each thread sums its samples in order and writes one partial image per
-// sample chunk; reduce_chunks adds the chunks in order, so the image is
-// deterministic.
+// pt_block: the paths of a block in lock step (block_paths.cuh), every scene
+// without subsurface materials; pixel sums in fixed point.
+//
+// pt_megakernel: one thread per (pixel, sample chunk), shadow rays and the
+// next segment traced in place, for subsurface scenes (whose frames live on
+// the thread's stack) and for pr_render_dev_noalloc (its 16 MiB hold no pool
+// of paths).  Each thread sums its samples in order and writes one partial
+// image per sample chunk; reduce_chunks adds the chunks in order.
+//
+// In both the refracted branch of a depth <= 2 glass split waits on a 4-entry
+// stack (at most three splits are pending at once: depths 0, 1, 2).
 #include <cuda_runtime.h>
 
 #include "path_logic.cuh"
@@ -132,8 +137,8 @@ __device__ float3 trace_sample(const DevScene& S, const RenderCfg& cfg, float3 o
 }
 
 // the lean form (no subsurface or glossy lobes) at 8 blocks of 128 per SM
-// (64 registers, spilling): plain mesh Cornell box 23.6 -> 24.8 Mpaths/s
-// on GB300; the fuller form keeps 3 blocks per SM (168 registers)
+// (64 registers, spilling): mesh Cornell box 23.6 -> 24.8 Mpaths/s on GB300;
+// the fuller forms keep 3 blocks per SM (168 registers)
 template <bool SSS, bool EXT>
 __global__ void __launch_bounds__(128, EXT ? 3 : 8) pt_megakernel(DevScene S, RenderCfg cfg, float* __restrict__ out,
                                                      uint32_t* __restrict__ err, unsigned long long* __restrict__ counters) {
@@ -181,7 +186,12 @@ __global__ void reduce_chunks(const float* __restrict__ partial, float* __restri
 // Resident blocks take camera samples one by one, pixel by pixel
 // (block_paths.cuh), and add each finished sample to its pixel in 64-bit
 // fixed point (2^-40: integer sums do not depend on the order in which
-// samples finish).
+// samples finish).  Bound by instruction issue and divergence; mesh Cornell
+// box 321x243 x 16 spp on GB300 37.7 ms in pt_megakernel, 8.5 here, spheres
+// 256x192 x 16 (FP64 sphere tests) 16.8 -> 6.9, Ward 404x248 x 4 22.2 -> 6.1.
+// FULL: glossy lobes, other lights, textures; the same shade() instantiations
+// as pt_megakernel's, since contraction (and with it a path's last bits)
+// differs between instantiations.
 struct PlainFrame {
   long long* pix;              // 3 per pixel
   unsigned long long* next;    // samples handed out

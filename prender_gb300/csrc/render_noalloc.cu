@@ -1,5 +1,6 @@
-// pr_render_dev_noalloc: the plain (megakernel) render for callers that must
-// not allocate device memory while they render.
+// pr_render_dev_noalloc: the plain render, one thread per pixel and sample
+// chunk (pt_megakernel), for callers that must not allocate device memory
+// while they render.
 //
 // Who needs it: frame loops with a hard time budget (cudaMalloc / cudaFree
 // can synchronise the whole device and stall the frame), and host
@@ -8,7 +9,7 @@
 // its accounting.  pr_render_dev grows its scratch on demand with
 // cudaMalloc; this entry point never does.
 //
-// Its scratch -- the per-chunk partial images of the megakernel and the
+// Its scratch -- the per-chunk partial images of that kernel and the
 // device error word / counters -- lives in one file-scope __device__ array
 // of kNoAllocScratchBytes (16 MiB), which every GPU that loads this library
 // keeps for the life of the process.  The first call on a device looks up
@@ -27,13 +28,11 @@
 // wrong images.  Each call clears the error word and counters it uses; the
 // partial images are fully overwritten by every call.
 //
-// Sample chunks: pr_render_dev splits each pixel's samples into
-// min(ceil(1.2e6 / pixels), spp) chunks, each summed by its own thread.
-// This entry point keeps that split while the chunks' partial images fit in
-// the array and otherwise uses as many chunks as fit (for example one
-// instead of two at 1024 x 768).  The samples are the same, only the order
-// of the float sums differs, so such images agree with pr_render_dev's to
-// float rounding, not bit for bit.
+// Sample chunks: each pixel's samples are split into min(ceil(1.2e6 / pixels),
+// spp) chunks, each summed by its own thread, or into as many as fit in the
+// array (for example one instead of two at 1024 x 768).  The samples are
+// pr_render_dev's, whose sums are in fixed point: images agree to float
+// rounding, not bit for bit.
 #include <cuda_runtime.h>
 
 #include <mutex>
