@@ -618,7 +618,8 @@ __device__ __forceinline__ bool warp_triangles(const DevScene& S, TraceLane& r, 
       hit = fast_tri(S.rtris + 3 * (size_t)slot, o, d, tmax, t, u, v);
       if (hit) found[lane] = make_float4(t, u, v, __int_as_float(slot));
     }
-    const uint32_t hits = __ballot_sync(0xffffffffu, hit);  // orders found[] too
+    const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+    __syncwarp();  // a vote orders no memory: the lanes' found[] before the reads of other lanes
     const int lo = max(excl - base, 0), hi = min(incl - base, 32);
     if (hits && hi > lo && !met) {
       uint32_t mine = hits & (0xffffffffu >> (32 - (hi - lo))) << lo;
@@ -640,7 +641,7 @@ __device__ __forceinline__ bool warp_triangles(const DevScene& S, TraceLane& r, 
         r.h.v = f.z;
       }
     }
-    __syncwarp();
+    __syncwarp();  // all reads before the next pairs' hits
   }
   if (!met) st.tris += cnt;
   return met;
