@@ -321,13 +321,13 @@ __device__ inline bool exact_qbvh(const DevScene& S, const GEntity& e, const Exa
   while (__any_sync(warp, sp > 0)) {
     uint32_t leaves = 0, order = 0;  // hit leaves and all children, in the reference's order
     const GNode* nd = S.nodes;
+    if (sp > 0 && ++guard > (1 << 24)) {  // a malformed tree: this lane visits no more
+      atomicOr(err, PR_DEV_LOOP_CAP);
+      sp = 0;
+    }
     if (sp > 0) {
       nd = S.nodes + stack[--sp];
       nodes_visited++;
-      if (++guard > (1 << 24)) {
-        atomicOr(err, PR_DEV_LOOP_CAP);
-        sp = 0;
-      }
       const float* lo[3] = {nd->bmin_x, nd->bmin_y, nd->bmin_z};
       const float* hi[3] = {nd->bmax_x, nd->bmax_y, nd->bmax_z};
       float tmin[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -364,6 +364,10 @@ __device__ inline bool exact_qbvh(const DevScene& S, const GEntity& e, const Exa
           atomicOr(err, PR_DEV_STACK_OVERFLOW);
           ok = false;
         }
+      }
+      if (!ok) {  // nor here
+        sp = 0;
+        leaves = 0;
       }
     }
     // the triangles of all hit leaves in one loop

@@ -1,6 +1,7 @@
 """Device code of prender_gb300/csrc compiled for the host (tests/host), where
 a fault may be shown that must not run on a GPU: accesses of shared memory
-between the lanes of a warp that no fence orders."""
+between the lanes of a warp that no fence orders, loops that only their caps
+end."""
 import os
 import shutil
 import subprocess
@@ -15,11 +16,11 @@ def _cuda_include():
     return os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build.nvcc()))), "include")
 
 
-def _run(tmp_path, name, flags=(), timeout=300):
+def _run(tmp_path, name, flags=(), args=(), timeout=300):
     exe = str(tmp_path / name)
     subprocess.run([shutil.which("g++"), "-std=c++17", "-O1", "-g", "-w", "-ffp-contract=off", "-pthread",
                     "-isystem", _cuda_include(), *flags, "-o", exe, os.path.join(HOST, name + ".cpp")], check=True)
-    return subprocess.run([exe], capture_output=True, text=True, timeout=timeout,
+    return subprocess.run([exe, *map(str, args)], capture_output=True, text=True, timeout=timeout,
                           env=dict(os.environ, TSAN_OPTIONS="exitcode=66 halt_on_error=1"))
 
 
@@ -29,3 +30,12 @@ def test_warp_triangles_is_each_lanes_own_loop_and_free_of_races(tmp_path, sanit
     if "FATAL: ThreadSanitizer" in r.stderr:  # this kernel's address layout is not one the sanitizer knows
         pytest.skip("the thread sanitizer does not start here")
     assert r.returncode == 0, r.stdout + r.stderr[-3000:]
+
+
+@pytest.mark.parametrize("kind,hit,err,nodes", [(0, 1, 0, 1), (1, 0, 2, 1 << 24), (2, 0, 1, 22)])
+def test_exact_traversal_of_a_malformed_tree_ends(tmp_path, kind, hit, err, nodes):
+    """err: PR_DEV_LOOP_CAP after 2^24 visits, PR_DEV_STACK_OVERFLOW where 64
+    entries, three more per visit, are full"""
+    r = _run(tmp_path, "exact_tree", ["-O2"], [kind], timeout=60)
+    got = [int(x) for x in r.stdout.split()]
+    assert got[0] == hit and got[2] == err and got[3] == nodes
