@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdlib>
 
 #include "adjoint.h"
 #include "block_paths.cuh"
@@ -259,25 +260,32 @@ __global__ void __launch_bounds__(128) adjoint_reduce(const __grid_constant__ Ad
 }
 
 constexpr size_t kAdjointBytes = 512ull << 20;  // of the samples of one pass (a lane's at most kAdjointLane)
-constexpr uint32_t kAdjointLane = 4096;
+constexpr uint32_t kAdjointLane = 4096;         // PR_ADJOINT_LANE may lower it
+
+uint32_t adjoint_lane() {
+  const char* e = getenv("PR_ADJOINT_LANE");
+  const long v = e ? strtol(e, nullptr, 10) : 0;
+  return v >= 1 && v < (long)kAdjointLane ? (uint32_t)v : kAdjointLane;
+}
 
 // warps and samples per lane of a pass, and the scratch it takes
 struct AdjointShape {
   uint32_t warps, pass_warps, lane_samples, kmax;  // kmax: a lane's samples in one pass
+  BlockShape blocks;                               // of the largest pass, for all of them
   size_t item_bytes, slot_bytes, slots, carry_bytes;
 };
 AdjointShape adjoint_shape(const RenderCfg& cfg, int n_mat) {
   AdjointShape h;
   h.warps = cfg.tiles_x * cfg.tiles_y * (uint32_t)cfg.chunks;
   h.lane_samples = (uint32_t)((cfg.spp + cfg.chunks - 1) / cfg.chunks);
-  h.kmax = std::min(h.lane_samples, kAdjointLane);
+  h.kmax = std::min(h.lane_samples, adjoint_lane());
   h.item_bytes = sizeof(float3) * (1 + 2 * (size_t)n_mat);
   const size_t per_warp = h.item_bytes * 32 * h.kmax;
   h.pass_warps = (uint32_t)std::max<size_t>(1, std::min<size_t>(h.warps, kAdjointBytes / per_warp));
-  const BlockShape b = block_shape((unsigned long long)h.pass_warps * 32 * h.kmax, sm_count());
-  h.slots = (size_t)b.blocks * b.slots;
+  h.blocks = block_shape((unsigned long long)h.pass_warps * 32 * h.kmax, sm_count());
+  h.slots = (size_t)h.blocks.blocks * h.blocks.slots;
   h.slot_bytes = sizeof(float4) * (n_mat + 3) + 4 + 8;
-  h.carry_bytes = h.lane_samples > h.kmax ? 24 * (size_t)n_mat * 32 * h.pass_warps : 0;
+  h.carry_bytes = h.lane_samples > h.kmax ? (24 * (size_t)n_mat * 32 * h.pass_warps + 255) / 256 * 256 : 0;
   return h;
 }
 
@@ -285,14 +293,16 @@ AdjointShape adjoint_shape(const RenderCfg& cfg, int n_mat) {
 
 size_t adjoint_scratch_bytes(const RenderCfg& cfg, int n_mat) {
   const AdjointShape h = adjoint_shape(cfg, n_mat);
-  return 256 + (h.item_bytes * h.pass_warps * 32 * h.kmax + 255) / 256 * 256 + block_pool_bytes(h.slots) +
-         (h.slot_bytes * h.slots + 255) / 256 * 256 + h.carry_bytes + 256;
+  return h.carry_bytes + 256 + (h.item_bytes * h.pass_warps * 32 * h.kmax + 255) / 256 * 256 +
+         block_pool_bytes(h.slots) + (h.slot_bytes * h.slots + 255) / 256 * 256 + 256;
 }
 
 cudaError_t launch_adjoint(const DevScene& S, const RenderCfg& cfg, const float* dl_drgb, int n_mat, void* scratch,
                            double* d_color, double* d_emission, uint32_t* err, unsigned long long* counters,
                            int* launches, cudaStream_t stream) {
   const AdjointShape h = adjoint_shape(cfg, n_mat);
+  const BlockShape& b = h.blocks;
+  const size_t n = h.slots;
   *launches = 0;
   for (uint32_t w0 = 0; w0 < h.warps; w0 += h.pass_warps)
     for (uint32_t k0 = 0; k0 < h.lane_samples; k0 += h.kmax) {
@@ -305,7 +315,10 @@ cudaError_t launch_adjoint(const DevScene& S, const RenderCfg& cfg, const float*
       A.last = k0 + A.kmax == h.lane_samples;
       A.items = (unsigned long long)warps * 32 * A.kmax;
       A.n_mat = n_mat;
-      char* p = static_cast<char*>(scratch);
+      // the carried sums come first, where every pass finds them: what follows
+      // is laid out by this pass's items, fewer in the last one
+      A.carry = static_cast<float*>(scratch);
+      char* p = static_cast<char*>(scratch) + h.carry_bytes;
       A.next = reinterpret_cast<unsigned long long*>(p);
       A.w = reinterpret_cast<float3*>(p + 256);
       A.g_col = A.w + A.items;
@@ -314,8 +327,6 @@ cudaError_t launch_adjoint(const DevScene& S, const RenderCfg& cfg, const float*
       cudaError_t e = cudaMemsetAsync(p, 0, zero, stream);
       if (e != cudaSuccess) return e;
       p += (zero + 255) / 256 * 256;
-      const BlockShape b = block_shape(A.items, sm_count());
-      const size_t n = (size_t)b.blocks * b.slots;
       BlockPool P = block_pool(p, n);
       P.slots = b.slots;
       P.slots_used = b.used;
@@ -324,7 +335,6 @@ cudaError_t launch_adjoint(const DevScene& S, const RenderCfg& cfg, const float*
       A.ew = A.acc + n * n_mat;
       A.item = reinterpret_cast<unsigned long long*>(A.ew + 3 * n);
       A.anc = reinterpret_cast<int*>(A.item + n);
-      A.carry = reinterpret_cast<float*>(p + (h.slot_bytes * n + 255) / 256 * 256);
       adjoint_paths<<<b.blocks, b.threads, block_shared_bytes(b), stream>>>(S, cfg, A, P, dl_drgb, err, counters);
       e = cudaGetLastError();
       if (e != cudaSuccess) return e;

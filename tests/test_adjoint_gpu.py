@@ -130,3 +130,19 @@ def test_adjoint_rejects_what_it_does_not_cover(ctx):
     ctx.upload(s)
     with pytest.raises(gpu.PrenderError):
         ctx.render_adjoint(np.zeros((12, 16, 3), np.float32), s)
+
+
+@pytest.mark.parametrize("samples,lane", [(1000, 2), (1000, 1), (1900, 2), (1900, 4)])
+def test_adjoint_passes_carry_a_lanes_sums(ctx, monkeypatch, samples, lane):
+    """A lane's samples (1000 / 391 chunks: up to 3, 1900: up to 5) in several
+    passes, the last one shorter, and lanes in two groups: the same FP32 sums
+    as in one pass, added up in FP64 in another order (1e5 warps' values)."""
+    s = scenes.diff_cornell(64, 48, samples=samples, supersamples=1, subdiv=3, seed=4)
+    ctx.upload(s)
+    dl = np.random.default_rng(6).uniform(0.5, 1.5, (48, 64, 3)).astype(np.float32)
+    whole = ctx.render_adjoint(dl)
+    monkeypatch.setenv("PR_ADJOINT_LANE", str(lane))
+    parts = ctx.render_adjoint(dl)
+    for key in ("color", "emission"):
+        assert np.abs(whole[key]).max() > 0.0
+        np.testing.assert_allclose(parts[key], whole[key], rtol=1e-9, atol=1e-9 * np.abs(whole[key]).max())
