@@ -1003,6 +1003,7 @@ struct KerrFar {
   Rng drng;
   PathState ps;
   float3 root;
+  uint32_t pixel;
   int c;
   int capture_checked;
 };
@@ -1036,6 +1037,7 @@ struct KerrPathJob {
   Rng drng;  // the accretion disk's alpha tests of this camera sample
   PathState ps;
   unsigned long long id;
+  uint32_t pixel;  // of the path (a sample id may wrap past 2^64)
   float3 L;
   int sp;
   uint32_t paths;
@@ -1084,6 +1086,7 @@ struct KerrPathJob {
       h.prim = -1;
       h.t = -1.0;
       id = f.id;
+      pixel = f.pixel;
       drng = f.drng;
       ps = f.ps;
       L = f.root;
@@ -1099,6 +1102,7 @@ struct KerrPathJob {
     const int y = (int)((uint32_t)px / (uint32_t)cfg.width), x = (int)((uint32_t)px - (uint32_t)y * cfg.width);
     float3 o, d;
     id = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
+    pixel = (uint32_t)(cfg.height - 1 - y) * (uint32_t)cfg.width + (uint32_t)x;
     root_path(ps, o, d);
     drng.init(disk_stream_key(cfg.seed, K), id, kDiskBranch);
     L = f3(0, 0, 0);
@@ -1129,6 +1133,7 @@ struct KerrPathJob {
           f.c = M.c;
           f.capture_checked = M.capture_checked;
           f.id = id;
+          f.pixel = pixel;
           f.drng = drng;
           f.ps = ps;
           f.root = L;
@@ -1194,9 +1199,7 @@ struct KerrPathJob {
       L += ps.L;
       if (sp == 0) {
         const float3 val = finish_sample(cfg, L, err);
-        const uint32_t p = (uint32_t)(id % ((unsigned long long)cfg.width * cfg.height));
-        const uint32_t y = p / (uint32_t)cfg.width, x = p - y * (uint32_t)cfg.width;
-        add_pixel(F.pix + 3 * ((size_t)(cfg.height - 1 - y) * cfg.width + x), val);
+        add_pixel(F.pix + 3 * (size_t)pixel, val);
         paths++;
         return false;
       }

@@ -196,6 +196,7 @@ struct PlainFrame {
   long long* pix;              // 3 per pixel
   unsigned long long* next;    // samples handed out
   unsigned long long samples;  // of the frame
+  uint32_t* pixel;             // per slot: the pixel of its path (a sample id may wrap past 2^64)
 };
 
 template <bool FULL>
@@ -228,6 +229,7 @@ struct PlainPaths {
     const int y = (int)((uint32_t)px / (uint32_t)cfg.width), x = (int)((uint32_t)px - (uint32_t)y * cfg.width);
     float3 o, d;
     P.id[i] = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
+    F.pixel[i] = (uint32_t)(cfg.height - 1 - y) * (uint32_t)cfg.width + (uint32_t)x;
     root_path(ps, o, d);
     return true;
   }
@@ -274,9 +276,7 @@ struct PlainPaths {
       }
     }
     const float3 v = finish_sample(cfg, L, err);
-    const uint32_t p = (uint32_t)(id % ((unsigned long long)cfg.width * cfg.height));
-    const uint32_t y = p / (uint32_t)cfg.width, x = p - y * (uint32_t)cfg.width;
-    add_pixel(F.pix + 3 * ((size_t)(cfg.height - 1 - y) * cfg.width + x), v);
+    add_pixel(F.pix + 3 * (size_t)F.pixel[i], v);
     paths++;
     return SHADE_END;
   }
@@ -315,7 +315,8 @@ static size_t pixel_bytes(const RenderCfg& cfg) { return (24 * (size_t)cfg.width
 
 size_t plain_scratch_bytes(const RenderCfg& cfg) {
   const BlockShape b = block_shape((unsigned long long)cfg.spp * cfg.width * cfg.height, sm_count());
-  return pixel_bytes(cfg) + block_pool_bytes((size_t)b.blocks * b.slots);
+  const size_t n = (size_t)b.blocks * b.slots;
+  return pixel_bytes(cfg) + (block_pool_bytes(n) + 255) / 256 * 256 + 4 * n;
 }
 
 cudaError_t launch_plain(const DevScene& S, const RenderCfg& cfg, void* scratch, float* dst, int accumulate,
@@ -328,7 +329,10 @@ cudaError_t launch_plain(const DevScene& S, const RenderCfg& cfg, void* scratch,
   cudaError_t e = cudaMemsetAsync(scratch, 0, pixel_bytes(cfg), stream);
   if (e != cudaSuccess) return e;
   const BlockShape b = block_shape(F.samples, sm_count());
-  BlockPool P = block_pool(static_cast<char*>(scratch) + pixel_bytes(cfg), (size_t)b.blocks * b.slots);
+  const size_t n = (size_t)b.blocks * b.slots;
+  char* p = static_cast<char*>(scratch) + pixel_bytes(cfg);
+  BlockPool P = block_pool(p, n);
+  F.pixel = reinterpret_cast<uint32_t*>(p + (block_pool_bytes(n) + 255) / 256 * 256);
   P.slots = b.slots;
   P.slots_used = b.used;
   const size_t smem = block_shared_bytes(b);

@@ -461,6 +461,7 @@ struct WormPathJob {
   WormCount c;
   PathState ps;
   unsigned long long id;
+  uint32_t pixel;  // of the path (a sample id may wrap past 2^64)
   float3 L;
   int sp;
   uint32_t paths;
@@ -486,6 +487,7 @@ struct WormPathJob {
     const int y = (int)((uint32_t)px / (uint32_t)cfg.width), x = (int)((uint32_t)px - (uint32_t)y * cfg.width);
     float3 o, d;
     id = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
+    pixel = (uint32_t)(cfg.height - 1 - y) * (uint32_t)cfg.width + (uint32_t)x;
     root_path(ps, o, d);
     L = f3(0, 0, 0);
     sp = 0;
@@ -540,9 +542,7 @@ struct WormPathJob {
       L += ps.L;
       if (sp == 0) {
         const float3 val = finish_sample(cfg, L, err);
-        const uint32_t p = (uint32_t)(id % ((unsigned long long)cfg.width * cfg.height));
-        const uint32_t y = p / (uint32_t)cfg.width, x = p - y * (uint32_t)cfg.width;
-        add_pixel(F.pix + 3 * ((size_t)(cfg.height - 1 - y) * cfg.width + x), val);
+        add_pixel(F.pix + 3 * (size_t)pixel, val);
         paths++;
         return false;
       }

@@ -92,3 +92,15 @@ def test_adjoint_of_two_sample_ranges_adds_up(ctx, w, h):
     for key in ("color", "emission"):
         both = parts[0][key] + parts[1][key]
         np.testing.assert_allclose(both, whole[key], rtol=1e-5, atol=1e-6 * np.abs(whole[key]).max() + 1e-30)
+
+
+@pytest.mark.parametrize("offset", [2 ** 60 + 1, 2 ** 63, 2 ** 64 - 2])
+@pytest.mark.parametrize("scene", ["spheres", "diffuse"])
+def test_block_form_equals_the_per_thread_form_far_along_the_streams(ctx, scene, offset):
+    """sample ids (offset x 33 x 17 + ...) wrap past 2^64: the streams go by
+    them, the pixels do not"""
+    if scene == "spheres":
+        s = scenes.cornell_spheres(33, 17, 1, 1)
+    else:
+        s = scenes.mesh_cornell(33, 17, 1, 1, subdiv=3)
+    _agree(*_both(ctx, s, offset=offset), 1)

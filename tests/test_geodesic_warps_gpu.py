@@ -62,3 +62,20 @@ def test_frames_are_the_sum_of_their_sample_ranges(ctx, kind, w, h):
     parts = ctx.render(s, settings=half) + ctx.render(s, settings=half, sample_offset=1)
     # two FP32 roundings of fixed-point sums
     np.testing.assert_allclose(parts, whole, rtol=4 * 2.0 ** -24, atol=2.0 ** -38)
+
+
+@pytest.mark.parametrize("kind", ["kerr64", "kerr32", "worm"])
+def test_frames_far_along_the_streams(ctx, kind):
+    """Sample ids (offset x pixels + ...) wrap past 2^64: frames whose rays
+    draw nothing are the same at any offset."""
+    if kind == "worm":
+        s = wormhole_cases.build("worm_bg", 37, 23, 1, 1, max_steps=60)
+    else:
+        s = scenes.kerr_lensing(a=0.9, width=37, height=23, max_steps=300)
+        s.kerr["precision"] = A.PR_KERR_FP32 if kind == "kerr32" else A.PR_KERR_FP64
+    s.settings = dataclasses.replace(s.settings, samples=1, supersamples=1, tent_filter=0)
+    ctx.upload(s)
+    near = ctx.render(s)
+    assert near.std() > 0.0
+    for offset in (2 ** 60 + 1, 2 ** 64 - 2):
+        assert np.array_equal(ctx.render(s, sample_offset=offset), near)
