@@ -934,6 +934,16 @@ static int render_wavefront(pr_ctx* c, const RenderCfg& g, float* rgb_dev, int a
   return PR_OK;
 }
 
+// the plain form of this scene is the block kernel (straight rays, no subsurface materials)
+static bool block_form(const SceneObjData& sc) { return !sc.kerr.enabled && !sc.worm.enabled && !sc.dev.has_sss; }
+
+// launches of a frame outside of the wavefront form: a kernel (two in the
+// mixed Kerr form) and the sum of every pass, or a subsurface scene's kernel and reduce
+static uint64_t frame_launches(const SceneObjData& sc, const RenderCfg& g) {
+  if (sc.kerr.enabled) return kerr_render_launches(sc.kerr, g);
+  return sc.worm.enabled || block_form(sc) ? 2 * pass_count(g) : 2;
+}
+
 int pr_render_dev(pr_ctx* c, const pr_camera* cam, const pr_render_params* p, float* rgb_dev, uint64_t sample_offset,
                   int accumulate) {
   if (!c) return PR_E_ARG;
@@ -989,9 +999,9 @@ int pr_render_dev(pr_ctx* c, const pr_camera* cam, const pr_render_params* p, fl
   const bool mlt = p->mode == PR_MODE_MLT && !kerr && !worm;
   // MLT: paths = bootstrap paths + proposals
   const uint64_t paths = wf ? (uint64_t)g.spp * g.width * g.height : mlt ? mlt_paths : cnt[0];
-  // wavefront: reset per pass + 4 per iteration + resolve; plain: kernel + resolve or reduce;
-  // MLT: bootstrap, chain start, the chains' launches, resolve
-  const uint64_t launches = wf ? 4 * cnt[5] + c->wf_passes + 1 : mlt ? mlt_launches : kerr ? (uint64_t)kerr_render_launches(c->cur.kerr) : 2;
+  // wavefront: reset per pass + 4 per iteration + resolve; MLT: bootstrap, chain
+  // start, the chains' launches, resolve; else frame_launches
+  const uint64_t launches = wf ? 4 * cnt[5] + c->wf_passes + 1 : mlt ? mlt_launches : frame_launches(c->cur, g);
   // Kerr counters: [1] accepted RK steps, [2] RK attempts, [3] segment scene
   // tests, reported as pr_kerr_trace does (segments, nodes_visited, tri_tests)
   c->stats = kerr ? pr_render_stats{paths, cnt[3], cnt[1], cnt[2], ms, launches}
@@ -1454,9 +1464,6 @@ int pr_kerr_sensitivity_adjoint(pr_ctx* c, const double* rays, int64_t n, const 
   return kerr_sens_common(c, rays, n, basis, cotangent, nullptr, nullptr, nullptr, grad);
 }
 
-// the plain form of this scene is the block kernel (straight rays, no subsurface materials)
-static bool block_form(const SceneObjData& sc) { return !sc.kerr.enabled && !sc.worm.enabled && !sc.dev.has_sss; }
-
 // Many jobs (scene object, camera, parameters, output) as one captured CUDA
 // graph: each job is the plain form (or a Kerr or wormhole frame) on its own
 // branch of the graph, so small and large frames overlap on the GPU; the graph is re-captured per call and updated
@@ -1581,7 +1588,7 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
   uint64_t launches = 0, wf_passes = 0;
   for (int j = 0; j < n; j++) {
     if (!wf_job[j]) {
-      launches += jobs[j].scene->data.kerr.enabled ? (uint64_t)kerr_render_launches(jobs[j].scene->data.kerr) : 2;
+      launches += frame_launches(jobs[j].scene->data, cfg[j]);
       continue;
     }
     const int stw = render_wavefront(c, cfg[j], jobs[j].rgb_dev, jobs[j].accumulate, &jobs[j].scene->data);

@@ -54,8 +54,10 @@ inline cudaError_t launch_kerr_trace(const DevScene& S, const GKerr& K, const do
 inline size_t kerr_scratch_bytes(const GKerr& K, const RenderCfg& cfg) {
   return K.precision == PR_KERR_FP32 ? kerr_scratch_bytes_fp32(cfg) : kerr_scratch_bytes_fp64(cfg);
 }
-// kernel and resolve; the mixed form's far field is a kernel of its own
-inline int kerr_render_launches(const GKerr& K) { return K.precision == PR_KERR_FP32 ? 3 : 2; }
+// kernel and sum of every pass; the mixed form's far field is a kernel of its own
+inline unsigned long long kerr_render_launches(const GKerr& K, const RenderCfg& cfg) {
+  return (K.precision == PR_KERR_FP32 ? 3 : 2) * pass_count(cfg);
+}
 inline cudaError_t launch_kerr_render(const DevScene& S, const GKerr& K, const RenderCfg& cfg, void* scratch, float* dst,
                                       int accumulate, uint32_t* err, unsigned long long* counters,
                                       cudaStream_t stream) {

@@ -17,21 +17,24 @@ cudaError_t launch_kerr_trace_fp32(const DevScene& S, const GKerr& K, const doub
   return cudaGetLastError();
 }
 
-size_t kerr_scratch_bytes_fp32(const RenderCfg& cfg) { return kerr_zero_bytes(cfg) + sizeof(KerrFar) * kerr_far_cap(cfg); }
+size_t kerr_scratch_bytes_fp32(const RenderCfg& cfg) { return kerr_bytes(cfg, true); }
 
 cudaError_t launch_kerr_render_fp32(const DevScene& S, const GKerr& K, const RenderCfg& cfg, void* scratch, float* dst,
                                     int accumulate, uint32_t* err, unsigned long long* counters, cudaStream_t stream) {
-  cudaError_t e = cudaMemsetAsync(scratch, 0, kerr_zero_bytes(cfg), stream);
-  if (e != cudaSuccess) return e;
-  const KerrFrame F = kerr_frame(cfg, scratch, true);
   const int sms = sm_count();
-  kerr_render_kernel<1><<<geodesic_blocks(F.samples, sms), 128, 0, stream>>>(S, K, cfg, F, err, counters);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  kerr_render_kernel<2><<<geodesic_blocks(F.far_cap, sms), 128, 0, stream>>>(S, K, cfg, F, err, counters);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  return launch_resolve(F.pix, dst, 3 * cfg.width * cfg.height, accumulate, cfg.sensor, stream);
+  for (unsigned long long k = 0, passes = pass_count(cfg); k < passes; k++) {
+    KerrFrame F;
+    cudaError_t e = kerr_frame(cfg, scratch, true, k, F, stream);
+    if (e != cudaSuccess) return e;
+    kerr_render_kernel<1><<<geodesic_blocks(F.pass.samples, sms), 128, 0, stream>>>(S, K, cfg, F, err, counters);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    kerr_render_kernel<2><<<geodesic_blocks(F.far_cap, sms), 128, 0, stream>>>(S, K, cfg, F, err, counters);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_sum(cfg, F.pass, dst, accumulate, stream);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace pr

@@ -1003,16 +1003,14 @@ struct KerrFar {
   Rng drng;
   PathState ps;
   float3 root;
-  uint32_t pixel;
+  uint32_t item;
   int c;
   int capture_checked;
 };
 
 struct KerrFrame {
-  long long* pix;              // 3 per pixel, fixed point (kPixelScaleF)
-  unsigned long long* next;    // [0] samples handed out, [1] far records written, [2] far records taken
-  unsigned long long samples;  // of the frame
-  KerrFar* far;                // mixed form
+  SamplePass pass;  // next: [0] samples handed out, [1] far records written, [2] far records taken
+  KerrFar* far;     // mixed form
   unsigned long long far_cap;
 };
 
@@ -1037,7 +1035,7 @@ struct KerrPathJob {
   Rng drng;  // the accretion disk's alpha tests of this camera sample
   PathState ps;
   unsigned long long id;
-  uint32_t pixel;  // of the path (a sample id may wrap past 2^64)
+  uint32_t item;  // the pass's sample that the path is (a sample id may wrap past 2^64)
   float3 L;
   int sp;
   uint32_t paths;
@@ -1057,13 +1055,13 @@ struct KerrPathJob {
     const unsigned int mask = __ballot_sync(0xffffffffu, want);
     const int leader = __ffs(mask) - 1;
     unsigned long long base = 0;
-    if (lane == leader) base = atomicAdd(F.next + (PHASE == 2 ? 2 : 0), (unsigned long long)__popc(mask));
+    if (lane == leader) base = atomicAdd(F.pass.next + (PHASE == 2 ? 2 : 0), (unsigned long long)__popc(mask));
     base = __shfl_sync(0xffffffffu, base, leader);
     if (!want) return false;
     const unsigned long long g = base + (unsigned long long)__popc(mask & ((1u << lane) - 1u));
     sp = 0;
     if (PHASE == 2) {
-      const unsigned long long n = F.next[1] < F.far_cap ? F.next[1] : F.far_cap;
+      const unsigned long long n = F.pass.next[1] < F.far_cap ? F.pass.next[1] : F.far_cap;
       if (g >= n) {
         more = false;
         return false;
@@ -1086,23 +1084,23 @@ struct KerrPathJob {
       h.prim = -1;
       h.t = -1.0;
       id = f.id;
-      pixel = f.pixel;
+      item = f.item;
       drng = f.drng;
       ps = f.ps;
       L = f.root;
       ended_at_start = false;
       return true;
     }
-    if (g >= F.samples) {
+    if (g >= F.pass.samples) {
       more = false;
       return false;
     }
-    const unsigned long long px = g / (unsigned int)cfg.spp;
-    const uint32_t k = (uint32_t)(g - px * (unsigned int)cfg.spp);
-    const int y = (int)((uint32_t)px / (uint32_t)cfg.width), x = (int)((uint32_t)px - (uint32_t)y * cfg.width);
+    int x, y;
+    uint32_t k;
+    pass_sample(cfg, F.pass, g, x, y, k);
     float3 o, d;
     id = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
-    pixel = (uint32_t)(cfg.height - 1 - y) * (uint32_t)cfg.width + (uint32_t)x;
+    item = (uint32_t)g;
     root_path(ps, o, d);
     drng.init(disk_stream_key(cfg.seed, K), id, kDiskBranch);
     L = f3(0, 0, 0);
@@ -1119,7 +1117,7 @@ struct KerrPathJob {
       // newly in the far field (or started a step there: no room in the list)
       if (run && !done && M.far_mode) {
         unsigned long long at = F.far_cap;
-        if (!far && sp == 0) at = atomicAdd(F.next + 1, 1ull);
+        if (!far && sp == 0) at = atomicAdd(F.pass.next + 1, 1ull);
         if (at < F.far_cap) {
           KerrFar& f = F.far[at];
           for (int q = 0; q < 6; q++) f.y[q] = M.y[q];
@@ -1133,7 +1131,7 @@ struct KerrPathJob {
           f.c = M.c;
           f.capture_checked = M.capture_checked;
           f.id = id;
-          f.pixel = pixel;
+          f.item = item;
           f.drng = drng;
           f.ps = ps;
           f.root = L;
@@ -1198,8 +1196,7 @@ struct KerrPathJob {
     if (r == SHADE_END) {
       L += ps.L;
       if (sp == 0) {
-        const float3 val = finish_sample(cfg, L, err);
-        add_pixel(F.pix + 3 * (size_t)pixel, val);
+        F.pass.sample[item] = finish_sample(cfg, L, err);
         paths++;
         return false;
       }
@@ -1227,22 +1224,20 @@ __global__ void __launch_bounds__(128) kerr_render_kernel(const __grid_constant_
   flush_counts(job.c, job.paths, counters);
 }
 
-// scratch of a frame: the pixel sums and counters (zeroed), the far records
-inline size_t kerr_zero_bytes(const RenderCfg& cfg) {
-  return (24 * (size_t)cfg.width * cfg.height + 32 + 255) / 256 * 256;
-}
+// scratch of a frame: the samples of a pass, then the far records
 inline unsigned long long kerr_far_cap(const RenderCfg& cfg) {
-  const unsigned long long n = (unsigned long long)cfg.spp * cfg.width * cfg.height;
+  const unsigned long long n = pass_pixels(cfg) * (unsigned long long)cfg.spp;
   return n < (1ull << 19) ? n : 1ull << 19;  // beyond that the near kernel goes on itself
 }
-inline KerrFrame kerr_frame(const RenderCfg& cfg, void* scratch, bool far) {
-  KerrFrame F;
-  F.pix = static_cast<long long*>(scratch);
-  F.next = reinterpret_cast<unsigned long long*>(F.pix + 3 * (size_t)cfg.width * cfg.height);
-  F.samples = (unsigned long long)cfg.spp * cfg.width * cfg.height;
-  F.far = far ? reinterpret_cast<KerrFar*>(static_cast<char*>(scratch) + kerr_zero_bytes(cfg)) : nullptr;
+inline size_t kerr_bytes(const RenderCfg& cfg, bool far) {
+  return pass_bytes(cfg) + (far ? sizeof(KerrFar) * (size_t)kerr_far_cap(cfg) : 0);
+}
+// pass k of a frame (its counters are zeroed)
+inline cudaError_t kerr_frame(const RenderCfg& cfg, void* scratch, bool far, unsigned long long k, KerrFrame& F,
+                              cudaStream_t stream) {
+  F.far = far ? reinterpret_cast<KerrFar*>(static_cast<char*>(scratch) + pass_bytes(cfg)) : nullptr;
   F.far_cap = far ? kerr_far_cap(cfg) : 0;
-  return F;
+  return sample_pass(cfg, scratch, k, F.pass, stream);
 }
 
 }  // namespace

@@ -3,7 +3,7 @@
 // the per-vertex logic of path_logic.cuh, in one kernel and in two shapes:
 //
 // pt_block: the paths of a block in lock step (block_paths.cuh), every scene
-// without subsurface materials; pixel sums in fixed point.
+// without subsurface materials; a pixel's samples added up by sum_samples.
 //
 // pt_megakernel: one thread per (pixel, sample chunk), shadow rays and the
 // next segment traced in place, for subsurface scenes (whose frames live on
@@ -184,19 +184,16 @@ __global__ void reduce_chunks(const float* __restrict__ partial, float* __restri
 
 // ---- the plain form without subsurface frames ------------------------------
 // Resident blocks take camera samples one by one, pixel by pixel
-// (block_paths.cuh), and add each finished sample to its pixel in 64-bit
-// fixed point (2^-40: integer sums do not depend on the order in which
-// samples finish).  Bound by instruction issue and divergence; mesh Cornell
+// (block_paths.cuh), and leave each finished sample in its place of the pass
+// (sum_samples adds them up).  Bound by instruction issue and divergence; mesh Cornell
 // box 321x243 x 16 spp on GB300 37.7 ms in pt_megakernel, 8.5 here, spheres
 // 256x192 x 16 (FP64 sphere tests) 16.8 -> 6.9, Ward 404x248 x 4 22.2 -> 6.1.
 // FULL: glossy lobes, other lights, textures; the same shade() instantiations
 // as pt_megakernel's, since contraction (and with it a path's last bits)
 // differs between instantiations.
 struct PlainFrame {
-  long long* pix;              // 3 per pixel
-  unsigned long long* next;    // samples handed out
-  unsigned long long samples;  // of the frame
-  uint32_t* pixel;             // per slot: the pixel of its path (a sample id may wrap past 2^64)
+  SamplePass pass;
+  uint32_t* item;  // per slot: the pass's sample that its path is (a sample id may wrap past 2^64)
 };
 
 template <bool FULL>
@@ -215,21 +212,21 @@ struct PlainPaths {
     if (!mask) return false;
     unsigned long long base = 0;
     const int leader = __ffs(mask) - 1;
-    if (lane == leader) base = atomicAdd(F.next, (unsigned long long)__popc(mask));
+    if (lane == leader) base = atomicAdd(F.pass.next, (unsigned long long)__popc(mask));
     base = __shfl_sync(0xffffffffu, base, leader);
     if (!((mask >> lane) & 1)) return false;
     const unsigned long long g = base + (unsigned long long)__popc(mask & ((1u << lane) - 1u));
-    if (g >= F.samples) {
+    if (g >= F.pass.samples) {
       more = false;
       return false;
     }
     // a pixel's samples one after another: the first segments of a warp are close together
-    const unsigned long long px = g / (unsigned int)cfg.spp;
-    const uint32_t k = (uint32_t)(g - px * (unsigned int)cfg.spp);
-    const int y = (int)((uint32_t)px / (uint32_t)cfg.width), x = (int)((uint32_t)px - (uint32_t)y * cfg.width);
+    int x, y;
+    uint32_t k;
+    pass_sample(cfg, F.pass, g, x, y, k);
     float3 o, d;
     P.id[i] = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
-    F.pixel[i] = (uint32_t)(cfg.height - 1 - y) * (uint32_t)cfg.width + (uint32_t)x;
+    F.item[i] = (uint32_t)g;
     root_path(ps, o, d);
     return true;
   }
@@ -275,8 +272,7 @@ struct PlainPaths {
         return SHADE_CONTINUE;
       }
     }
-    const float3 v = finish_sample(cfg, L, err);
-    add_pixel(F.pix + 3 * (size_t)F.pixel[i], v);
+    F.pass.sample[F.item[i]] = finish_sample(cfg, L, err);
     paths++;
     return SHADE_END;
   }
@@ -295,54 +291,88 @@ __global__ void __launch_bounds__(kBlockThreads, 1)
   if (counters) add_counters(counters, drv.paths, segs, st);
 }
 
-// fixed-point pixel sums -> float image times the sensor response
-// (render.h:1405-1409); accumulate != 0 adds to what dst holds
-__global__ void resolve_pixels(const long long* __restrict__ pix, float* __restrict__ dst, int n3, int accumulate,
-                               float sensor) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n3) return;
-  const float v = __ll2float_rn(pix[i]) * kPixelInvF * sensor;
-  dst[i] = accumulate ? dst[i] + v : v;
+// Adds up the samples of n pixels from px0 on, g threads a pixel (a power of
+// two up to 32, or the whole block), times the sensor response
+// (render.h:1405-1409); accumulate != 0 adds to what dst holds.  12 bytes a
+// sample: 64 spp of 1024x768 in 0.2 ms of the frame's 360.
+constexpr int kSumThreads = 256;
+__global__ void __launch_bounds__(kSumThreads)
+    sum_samples(const float3* __restrict__ sample, float* __restrict__ dst, int width, int height, uint32_t spp,
+                unsigned long long px0, unsigned long long n, uint32_t g, int accumulate, float sensor) {
+  __shared__ double part[kSumThreads / 32][3];
+  const unsigned long long t = (unsigned long long)blockIdx.x * kSumThreads + threadIdx.x, p = t / g;
+  const uint32_t l = (uint32_t)(t - p * g);
+  double a[3] = {0.0, 0.0, 0.0};
+  if (p < n)
+    for (uint32_t k = l; k < spp; k += g) {
+      const float3 v = sample[p * spp + k];
+      a[0] += (double)v.x;
+      a[1] += (double)v.y;
+      a[2] += (double)v.z;
+    }
+  for (int off = (int)(g < 32 ? g : 32) / 2; off > 0; off >>= 1)
+#pragma unroll
+    for (int c = 0; c < 3; c++) a[c] += __shfl_down_sync(0xffffffffu, a[c], off);
+  if (g > 32) {
+    if ((threadIdx.x & 31) == 0)
+      for (int c = 0; c < 3; c++) part[threadIdx.x / 32][c] = a[c];
+    __syncthreads();
+    for (int w = 1; w < kSumThreads / 32; w++)
+      for (int c = 0; c < 3; c++) a[c] += part[w][c];
+  }
+  if (p >= n || l != 0) return;
+  const unsigned long long px = px0 + p, y = px / (unsigned int)width, x = px - y * (unsigned int)width;
+  float* o = dst + 3 * ((size_t)(height - 1 - (int)y) * width + (size_t)x);
+  for (int c = 0; c < 3; c++) {
+    const float v = (float)a[c] * sensor;
+    o[c] = accumulate ? o[c] + v : v;
+  }
 }
 
-cudaError_t launch_resolve(const long long* pix, float* dst, int n3, int accumulate, float sensor, cudaStream_t stream) {
-  resolve_pixels<<<(n3 + 255) / 256, 256, 0, stream>>>(pix, dst, n3, accumulate, sensor);
+cudaError_t launch_sum(const RenderCfg& cfg, const SamplePass& A, float* dst, int accumulate, cudaStream_t stream) {
+  const uint32_t spp = (uint32_t)cfg.spp;
+  uint32_t g = 1;  // from 1024 samples a pixel on a block each: a warp alone would take them in 32 or more rounds
+  while (g < 32 && 2 * g <= spp) g *= 2;
+  if (spp >= 1024) g = kSumThreads;
+  const unsigned long long n = A.samples / spp, blocks = (n * g + kSumThreads - 1) / kSumThreads;
+  sum_samples<<<(unsigned)blocks, kSumThreads, 0, stream>>>(A.sample, dst, cfg.width, cfg.height, spp, A.px0, n, g,
+                                                            accumulate, cfg.sensor);
   return cudaGetLastError();
 }
 
-// scratch: the pixel sums and the sample counter (zeroed by the launch), then the pool
-static size_t pixel_bytes(const RenderCfg& cfg) { return (24 * (size_t)cfg.width * cfg.height + 16 + 255) / 256 * 256; }
+// blocks of the frame's largest pass, for all of its passes
+static BlockShape plain_shape(const RenderCfg& cfg) {
+  return block_shape(pass_pixels(cfg) * (unsigned long long)cfg.spp, sm_count());
+}
 
 size_t plain_scratch_bytes(const RenderCfg& cfg) {
-  const BlockShape b = block_shape((unsigned long long)cfg.spp * cfg.width * cfg.height, sm_count());
+  const BlockShape b = plain_shape(cfg);
   const size_t n = (size_t)b.blocks * b.slots;
-  return pixel_bytes(cfg) + (block_pool_bytes(n) + 255) / 256 * 256 + 4 * n;
+  return pass_bytes(cfg) + (block_pool_bytes(n) + 255) / 256 * 256 + 4 * n;
 }
 
 cudaError_t launch_plain(const DevScene& S, const RenderCfg& cfg, void* scratch, float* dst, int accumulate,
                          uint32_t* err, unsigned long long* counters, cudaStream_t stream) {
-  const size_t n3 = 3 * (size_t)cfg.width * cfg.height;
-  PlainFrame F;
-  F.pix = static_cast<long long*>(scratch);
-  F.next = reinterpret_cast<unsigned long long*>(F.pix + n3);
-  F.samples = (unsigned long long)cfg.spp * cfg.width * cfg.height;
-  cudaError_t e = cudaMemsetAsync(scratch, 0, pixel_bytes(cfg), stream);
-  if (e != cudaSuccess) return e;
-  const BlockShape b = block_shape(F.samples, sm_count());
-  const size_t n = (size_t)b.blocks * b.slots;
-  char* p = static_cast<char*>(scratch) + pixel_bytes(cfg);
+  const BlockShape b = plain_shape(cfg);
+  const size_t n = (size_t)b.blocks * b.slots, smem = block_shared_bytes(b);
+  char* p = static_cast<char*>(scratch) + pass_bytes(cfg);
   BlockPool P = block_pool(p, n);
-  F.pixel = reinterpret_cast<uint32_t*>(p + (block_pool_bytes(n) + 255) / 256 * 256);
   P.slots = b.slots;
   P.slots_used = b.used;
-  const size_t smem = block_shared_bytes(b);
-  if (S.has_glossy || S.n_point_lights > 0 || S.has_tex)
-    pt_block<true><<<b.blocks, b.threads, smem, stream>>>(S, cfg, F, P, err, counters);
-  else
-    pt_block<false><<<b.blocks, b.threads, smem, stream>>>(S, cfg, F, P, err, counters);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  return launch_resolve(F.pix, dst, (int)n3, accumulate, cfg.sensor, stream);
+  PlainFrame F;
+  F.item = reinterpret_cast<uint32_t*>(p + (block_pool_bytes(n) + 255) / 256 * 256);
+  for (unsigned long long k = 0, passes = pass_count(cfg); k < passes; k++) {
+    cudaError_t e = sample_pass(cfg, scratch, k, F.pass, stream);
+    if (e != cudaSuccess) return e;
+    if (S.has_glossy || S.n_point_lights > 0 || S.has_tex)
+      pt_block<true><<<b.blocks, b.threads, smem, stream>>>(S, cfg, F, P, err, counters);
+    else
+      pt_block<false><<<b.blocks, b.threads, smem, stream>>>(S, cfg, F, P, err, counters);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_sum(cfg, F.pass, dst, accumulate, stream);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t launch_megakernel(const DevScene& S, const RenderCfg& cfg, float* out, uint32_t* err,

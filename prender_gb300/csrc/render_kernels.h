@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstdlib>
 
 #include "pr_internal.h"
 
@@ -27,20 +28,57 @@ struct RenderCfg {
   uint64_t sample_offset;
 };
 
-// Pixel sums in 64-bit fixed point (2^-40): integer sums do not depend on the
-// order in which samples finish.
-constexpr float kPixelScaleF = 1099511627776.0f;  // 2^40
-constexpr float kPixelInvF = 1.0f / 1099511627776.0f;
+// A frame whose samples finish in any order (plain form, Kerr and wormhole
+// frames): each leaves its radiance in its own place, pixel by pixel, and
+// sum_samples adds up a pixel's samples in FP64 in a fixed order, so the image
+// does not depend on the schedule and holds any finite value (sums in fixed
+// point wrap or lose what lies outside of their range).  A frame of more
+// samples than kPassSamples takes passes of whole pixels.
+struct SamplePass {
+  float3* sample;              // samples of the pass's pixels, one pixel after another
+  unsigned long long* next;    // samples handed out (and the callers' own counters, 256 bytes, zero at the start)
+  unsigned long long samples;  // of the pass
+  unsigned long long px0;      // its first pixel (scan line order)
+};
+// 192 MB of samples; PR_PASS_SAMPLES may lower it
+constexpr unsigned long long kPassSamples = 1ull << 24;
+inline unsigned long long pass_pixels(const RenderCfg& cfg) {
+  const char* e = getenv("PR_PASS_SAMPLES");
+  const long long v = e ? strtoll(e, nullptr, 10) : 0;
+  const unsigned long long most = v >= 1 && v < (long long)kPassSamples ? (unsigned long long)v : kPassSamples;
+  const unsigned long long px = (unsigned long long)cfg.width * cfg.height, n = most / (unsigned long long)cfg.spp;
+  return n < 1 ? 1 : n < px ? n : px;
+}
+inline unsigned long long pass_count(const RenderCfg& cfg) {
+  const unsigned long long px = (unsigned long long)cfg.width * cfg.height, n = pass_pixels(cfg);
+  return (px + n - 1) / n;
+}
+// a frame's counters and samples, ahead of the callers' own scratch
+inline size_t pass_bytes(const RenderCfg& cfg) {
+  return 256 + (sizeof(float3) * (size_t)pass_pixels(cfg) * (size_t)cfg.spp + 255) / 256 * 256;
+}
+// pass k; its counters are zeroed on the stream
+inline cudaError_t sample_pass(const RenderCfg& cfg, void* scratch, unsigned long long k, SamplePass& A,
+                               cudaStream_t stream) {
+  const unsigned long long px = (unsigned long long)cfg.width * cfg.height, n = pass_pixels(cfg);
+  A.next = static_cast<unsigned long long*>(scratch);
+  A.sample = reinterpret_cast<float3*>(static_cast<char*>(scratch) + 256);
+  A.px0 = k * n;
+  A.samples = (px - A.px0 < n ? px - A.px0 : n) * (unsigned long long)cfg.spp;
+  return cudaMemsetAsync(scratch, 0, 256, stream);
+}
+// the pass's pixels -> float image times the sensor response; accumulate adds to it
+cudaError_t launch_sum(const RenderCfg& cfg, const SamplePass& A, float* dst, int accumulate, cudaStream_t stream);
 #ifdef __CUDACC__
-__device__ __forceinline__ void add_pixel(long long* pix, float3 v) {
-  unsigned long long* p = reinterpret_cast<unsigned long long*>(pix);
-  atomicAdd(p + 0, (unsigned long long)__float2ll_rn(v.x * kPixelScaleF));
-  atomicAdd(p + 1, (unsigned long long)__float2ll_rn(v.y * kPixelScaleF));
-  atomicAdd(p + 2, (unsigned long long)__float2ll_rn(v.z * kPixelScaleF));
+// pixel and sample of the pass's sample g
+__device__ __forceinline__ void pass_sample(const RenderCfg& cfg, const SamplePass& A, unsigned long long g, int& x,
+                                            int& y, uint32_t& k) {
+  const unsigned long long p = g / (unsigned int)cfg.spp, px = A.px0 + p;
+  k = (uint32_t)(g - p * (unsigned int)cfg.spp);
+  y = (int)((uint32_t)px / (uint32_t)cfg.width);
+  x = (int)((uint32_t)px - (uint32_t)y * (uint32_t)cfg.width);
 }
 #endif
-// pixel sums -> float image times the sensor response; accumulate adds to it
-cudaError_t launch_resolve(const long long* pix, float* dst, int n3, int accumulate, float sensor, cudaStream_t stream);
 // SMs of the current device
 inline int sm_count() {
   int dev = 0, sms = 0;
@@ -54,8 +92,8 @@ cudaError_t launch_megakernel(const DevScene& S, const RenderCfg& cfg, float* ou
                               unsigned long long* counters, cudaStream_t stream);
 cudaError_t launch_reduce(const float* partial, float* dst, int n3, int chunks, int accumulate, cudaStream_t stream);
 // the plain form of scenes without subsurface materials: one kernel and the
-// resolve into dst; scratch (plain_scratch_bytes) holds the pixel sums
-// and the blocks' path slots
+// sum into dst per pass; scratch (plain_scratch_bytes) holds the samples and
+// the blocks' path slots
 size_t plain_scratch_bytes(const RenderCfg& cfg);
 cudaError_t launch_plain(const DevScene& S, const RenderCfg& cfg, void* scratch, float* dst, int accumulate,
                           uint32_t* err, unsigned long long* counters, cudaStream_t stream);

@@ -438,12 +438,6 @@ __global__ void __launch_bounds__(128) worm_trace_kernel(const __grid_constant__
   }
 }
 
-struct WormFrame {
-  long long* pix;              // 3 per pixel, fixed point (kPixelScaleF)
-  unsigned long long* next;    // samples handed out
-  unsigned long long samples;  // of the frame
-};
-
 // Camera samples of radiance() in a wormhole scene, one path per lane (no
 // next-event estimation, no media: every query goes through the wormhole).
 // Objects on the far side sit more than 1e6 from the origin (the trace picks
@@ -454,14 +448,14 @@ struct WormPathJob {
   const DevScene& S;
   const GWorm& W;
   const RenderCfg& cfg;
-  const WormFrame& F;
+  const SamplePass& F;
   uint32_t* err;
   WormMarch M;
   WormHit h;
   WormCount c;
   PathState ps;
   unsigned long long id;
-  uint32_t pixel;  // of the path (a sample id may wrap past 2^64)
+  uint32_t item;  // the pass's sample that the path is (a sample id may wrap past 2^64)
   float3 L;
   int sp;
   uint32_t paths;
@@ -482,12 +476,12 @@ struct WormPathJob {
       more = false;
       return false;
     }
-    const unsigned long long px = g / (unsigned int)cfg.spp;
-    const uint32_t k = (uint32_t)(g - px * (unsigned int)cfg.spp);
-    const int y = (int)((uint32_t)px / (uint32_t)cfg.width), x = (int)((uint32_t)px - (uint32_t)y * cfg.width);
+    int x, y;
+    uint32_t k;
+    pass_sample(cfg, F, g, x, y, k);
     float3 o, d;
     id = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
-    pixel = (uint32_t)(cfg.height - 1 - y) * (uint32_t)cfg.width + (uint32_t)x;
+    item = (uint32_t)g;
     root_path(ps, o, d);
     L = f3(0, 0, 0);
     sp = 0;
@@ -541,8 +535,7 @@ struct WormPathJob {
     if (r == SHADE_END) {
       L += ps.L;
       if (sp == 0) {
-        const float3 val = finish_sample(cfg, L, err);
-        add_pixel(F.pix + 3 * (size_t)pixel, val);
+        F.sample[item] = finish_sample(cfg, L, err);
         paths++;
         return false;
       }
@@ -558,7 +551,7 @@ struct WormPathJob {
 __global__ void __launch_bounds__(128) worm_render_kernel(const __grid_constant__ DevScene S,
                                                           const __grid_constant__ GWorm W,
                                                           const __grid_constant__ RenderCfg cfg,
-                                                          const __grid_constant__ WormFrame F,
+                                                          const __grid_constant__ SamplePass F,
                                                           uint32_t* __restrict__ err,
                                                           unsigned long long* __restrict__ counters) {
   WormPathJob job{S, W, cfg, F, err};
@@ -594,20 +587,20 @@ cudaError_t launch_worm_trace(const DevScene& S, const GWorm& W, const double* r
   return cudaGetLastError();
 }
 
-size_t worm_scratch_bytes(const RenderCfg& cfg) { return 24 * (size_t)cfg.width * cfg.height + 16; }
+size_t worm_scratch_bytes(const RenderCfg& cfg) { return pass_bytes(cfg); }
 
 cudaError_t launch_worm_render(const DevScene& S, const GWorm& W, const RenderCfg& cfg, void* scratch, float* dst,
                                int accumulate, uint32_t* err, unsigned long long* counters, cudaStream_t stream) {
-  cudaError_t e = cudaMemsetAsync(scratch, 0, worm_scratch_bytes(cfg), stream);
-  if (e != cudaSuccess) return e;
-  WormFrame F;
-  F.pix = static_cast<long long*>(scratch);
-  F.next = reinterpret_cast<unsigned long long*>(F.pix + 3 * (size_t)cfg.width * cfg.height);
-  F.samples = (unsigned long long)cfg.spp * cfg.width * cfg.height;
-  worm_render_kernel<<<geodesic_blocks(F.samples, sm_count()), 128, 0, stream>>>(S, W, cfg, F, err, counters);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  return launch_resolve(F.pix, dst, 3 * cfg.width * cfg.height, accumulate, cfg.sensor, stream);
+  for (unsigned long long k = 0, passes = pass_count(cfg); k < passes; k++) {
+    SamplePass F;
+    cudaError_t e = sample_pass(cfg, scratch, k, F, stream);
+    if (e != cudaSuccess) return e;
+    worm_render_kernel<<<geodesic_blocks(F.samples, sm_count()), 128, 0, stream>>>(S, W, cfg, F, err, counters);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_sum(cfg, F, dst, accumulate, stream);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace pr

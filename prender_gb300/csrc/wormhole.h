@@ -23,7 +23,7 @@ cudaError_t launch_worm_trace(const DevScene& S, const GWorm& W, const double* r
                               uint32_t* err, unsigned long long* counters, cudaStream_t stream);
 
 // the renderer with every scene query traced through the wormhole, into dst
-// (scratch of worm_scratch_bytes): a kernel and the resolve
+// (scratch of worm_scratch_bytes): a kernel and the sum of every pass
 size_t worm_scratch_bytes(const RenderCfg& cfg);
 cudaError_t launch_worm_render(const DevScene& S, const GWorm& W, const RenderCfg& cfg, void* scratch, float* dst,
                                int accumulate, uint32_t* err, unsigned long long* counters, cudaStream_t stream);
