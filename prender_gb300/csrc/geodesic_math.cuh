@@ -98,6 +98,7 @@ __device__ __forceinline__ int segment_draws(const DevScene& S, dv3 org, dv3 dir
   const float mo = fmaxf(fabsf(o.x), fmaxf(fabsf(o.y), fabsf(o.z)));
   const float dl = sqrtf(dot(d, d));
   const float reach = (float)within * dl;
+  const bool unit = fabsf(dl - 1.0f) < 1.0e-6f;
   int draws = 0;
   bool need = false;
   for (int i = 0; i < S.n_ents; i++) {
@@ -106,10 +107,13 @@ __device__ __forceinline__ int segment_draws(const DevScene& S, dv3 org, dv3 dir
     const float mw = fmaxf(fabsf(w.x), fmaxf(fabsf(w.y), fabsf(w.z)));
     const float tol = 4.0e-6f * (2.0f * mo + mw + reach) + 1.0e-4f;
     if (e.type == PR_ENT_SPHERE) {
-      // | |w| - r | > reach + tol, squared: no root
-      const float r = e.radius_eps, q = reach + tol + 1.0e-5f * r, w2 = dot(w, w);
+      // | |w| - r | > reach + tol, squared: no root.  The test's quadratic has
+      // |d| = 1: with another length its roots are not where the line meets the
+      // sphere, and a length off by e (FP32 cannot tell 1e-6) moves them by up
+      // to sqrt(2 e) of the segment, where the line goes through a small sphere
+      const float r = e.radius_eps, q = 1.002f * reach + tol + 1.0e-5f * r, w2 = dot(w, w);
       const float hi = r + q, lo = fmaxf(r - q, 0.0f);
-      need = need || !(w2 > hi * hi * 1.00001f || w2 < lo * lo * 0.99999f);
+      need = need || !unit || !(w2 > hi * hi * 1.00001f || w2 < lo * lo * 0.99999f);
     } else if (e.type == PR_ENT_UVPLANE || e.type == PR_ENT_CIRCLE) {
       const float3 n = f3(e.n[0], e.n[1], e.n[2]);
       const float nl = sqrtf(dot(n, n)), num = dot(w, n), den = dot(d, n);

@@ -69,7 +69,6 @@ inline cudaError_t sample_pass(const RenderCfg& cfg, void* scratch, unsigned lon
 }
 // the pass's pixels -> float image times the sensor response; accumulate adds to it
 cudaError_t launch_sum(const RenderCfg& cfg, const SamplePass& A, float* dst, int accumulate, cudaStream_t stream);
-#ifdef __CUDACC__
 // pixel and sample of the pass's sample g
 __device__ __forceinline__ void pass_sample(const RenderCfg& cfg, const SamplePass& A, unsigned long long g, int& x,
                                             int& y, uint32_t& k) {
@@ -78,7 +77,6 @@ __device__ __forceinline__ void pass_sample(const RenderCfg& cfg, const SamplePa
   y = (int)((uint32_t)px / (uint32_t)cfg.width);
   x = (int)((uint32_t)px - (uint32_t)y * (uint32_t)cfg.width);
 }
-#endif
 // SMs of the current device
 inline int sm_count() {
   int dev = 0, sms = 0;

@@ -65,6 +65,9 @@ struct HostThreadIdx {
   } x;
 };
 inline HostThreadIdx threadIdx;
+inline constexpr host::Index blockIdx{0, 0, 0}, blockDim{32, 1, 1}, gridDim{1, 1, 1};
+#define __launch_bounds__(...)
+#define __global__ static
 
 inline unsigned int __ballot_sync(unsigned int, int p) {
   uint32_t v[host::kMaxLanes];
@@ -77,16 +80,22 @@ inline int __any_sync(unsigned int m, int p) { return __ballot_sync(m, p) != 0; 
 inline unsigned int __activemask() { return host::lanes == 32 ? 0xffffffffu : (1u << host::lanes) - 1u; }
 template <class T>
 T __shfl_sync(unsigned int, T x, int src) {
-  static_assert(sizeof(T) == 4, "32-bit shuffles");
-  uint32_t b, v[host::kMaxLanes];
-  memcpy(&b, &x, 4);
-  host::exchange(b, v);
-  memcpy(&x, &v[src & 31], 4);
+  uint32_t b[sizeof(T) / 4], v[host::kMaxLanes];
+  memcpy(b, &x, sizeof(T));
+  for (uint32_t& w : b) {
+    host::exchange(w, v);
+    w = v[src & 31];
+  }
+  memcpy(&x, b, sizeof(T));
   return x;
 }
 template <class T>
 T __shfl_up_sync(unsigned int m, T x, int d) {
   return __shfl_sync(m, x, host::lane >= d ? host::lane - d : host::lane);
+}
+template <class T>
+T __shfl_down_sync(unsigned int m, T x, int d) {
+  return __shfl_sync(m, x, host::lane + d < host::lanes ? host::lane + d : host::lane);
 }
 inline void __syncwarp() {
   if (host::lanes == 1) return;
@@ -133,6 +142,10 @@ inline float rsqrtf(float x) { return 1.0f / sqrtf(x); }
 template <class T>
 T __ldg(const T* p) { return *p; }
 inline unsigned int atomicOr(unsigned int* p, unsigned int v) { return __atomic_fetch_or(p, v, __ATOMIC_RELAXED); }
+inline unsigned int atomicAdd(unsigned int* p, unsigned int v) { return __atomic_fetch_add(p, v, __ATOMIC_RELAXED); }
+inline unsigned long long atomicAdd(unsigned long long* p, unsigned long long v) {
+  return __atomic_fetch_add(p, v, __ATOMIC_RELAXED);
+}
 inline int min(int a, int b) { return a < b ? a : b; }
 inline int max(int a, int b) { return a > b ? a : b; }
 inline unsigned int min(unsigned int a, unsigned int b) { return a < b ? a : b; }

@@ -39,3 +39,11 @@ def test_exact_traversal_of_a_malformed_tree_ends(tmp_path, kind, hit, err, node
     r = _run(tmp_path, "exact_tree", ["-O2"], [kind], timeout=60)
     got = [int(x) for x in r.stdout.split()]
     assert got[0] == hit and got[2] == err and got[3] == nodes
+
+
+@pytest.mark.parametrize("length", [1.0, 1.0 + 4e-7, 1.0 - 4e-7, 1.0 + 3e-6, 0.5, 0.9, 2.0, 10.0])
+def test_segments_left_out_have_no_hit(tmp_path, length):
+    """the sphere test takes directions for unit vectors: with others it has
+    roots where the line meets nothing"""
+    r = _run(tmp_path, "segment_tests", ["-O2"], [length])
+    assert r.returncode == 0, r.stdout + r.stderr[-3000:]
