@@ -47,3 +47,10 @@ def test_segments_left_out_have_no_hit(tmp_path, length):
     roots where the line meets nothing"""
     r = _run(tmp_path, "segment_tests", ["-O2"], [length])
     assert r.returncode == 0, r.stdout + r.stderr[-3000:]
+
+
+@pytest.mark.parametrize("length", [1.0, 0.7, 3.0])
+@pytest.mark.parametrize("scene", ["walls", "nested", "hemispheres", "many"])
+def test_sphere_runs_are_the_fp64_tests_of_every_sphere(tmp_path, scene, length):
+    r = _run(tmp_path, "sphere_runs", ["-O2"], [scene, length])
+    assert r.returncode == 0, r.stdout + r.stderr[-3000:]
