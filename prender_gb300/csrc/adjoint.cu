@@ -281,8 +281,8 @@ AdjointShape adjoint_shape(const RenderCfg& cfg, int n_mat) {
   h.kmax = std::min(h.lane_samples, adjoint_lane());
   h.item_bytes = sizeof(float3) * (1 + 2 * (size_t)n_mat);
   const size_t per_warp = h.item_bytes * 32 * h.kmax;
-  h.pass_warps = (uint32_t)std::max<size_t>(1, std::min<size_t>(h.warps, kAdjointBytes / per_warp));
-  h.blocks = block_shape((unsigned long long)h.pass_warps * 32 * h.kmax, sm_count());
+  h.pass_warps = (uint32_t)std::max<size_t>(1, std::min<size_t>(h.warps, (cfg.less ? kAdjointBytes / 16 : kAdjointBytes) / per_warp));
+  h.blocks = block_shape((unsigned long long)h.pass_warps * 32 * h.kmax, slot_sms(cfg));
   h.slots = (size_t)h.blocks.blocks * h.blocks.slots;
   h.slot_bytes = sizeof(float4) * (n_mat + 3) + 4 + 8;
   h.carry_bytes = h.lane_samples > h.kmax ? (24 * (size_t)n_mat * 32 * h.pass_warps + 255) / 256 * 256 : 0;

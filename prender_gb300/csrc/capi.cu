@@ -328,6 +328,7 @@ static int build_device_scene(pr_ctx* c, const pr_scene_desc* d, SceneObjData& o
 int pr_scene_upload(pr_ctx* c, const pr_scene_desc* d) {
   if (!c) return PR_E_ARG;
   c->scene_ready = false;
+  c->less_memory = false;
   int st = build_device_scene(c, d, c->cur);
   if (st != PR_OK) return st;
   c->scene_ready = true;
@@ -358,6 +359,7 @@ pr_scene_obj* pr_scene_create(pr_ctx* c, const pr_scene_desc* d, int* status) {
     if (status) *status = PR_E_ARG;
     return nullptr;
   }
+  c->less_memory = false;
   pr_scene_obj* o = new pr_scene_obj();
   int st = build_device_scene(c, d, o->data);
   if (status) *status = st;
@@ -627,7 +629,22 @@ int pr::prepare_render(pr_ctx* c, const pr_camera* cam, const pr_render_params* 
   int chunks = (int)std::ceil(1.2e6 / pixels);
   chunks = std::max(1, std::min(chunks, g.spp));
   g.chunks = chunks;
+  g.less = c->less_memory ? 1 : 0;
   return PR_OK;
+}
+
+// Grows a frame's scratch to bytes(g); where the device cannot hold that, to
+// the sizes of little memory (g.less), which the context then keeps to until
+// the next scene upload or object: another try in every frame would free and
+// allocate anew.
+template <class Bytes>
+static cudaError_t ensure_scratch(pr_ctx* c, RenderCfg& g, DevBuf& b, Bytes bytes) {
+  cudaError_t e = b.ensure(bytes(g));
+  if (e != cudaErrorMemoryAllocation || g.less) return e;
+  cudaGetLastError();
+  c->less_memory = true;
+  g.less = 1;
+  return b.ensure(bytes(g));
 }
 
 extern "C" {
@@ -687,7 +704,7 @@ static int render_mlt(pr_ctx* c, const RenderCfg& g0, const pr_render_params* p,
   PR_CUDA(c, c->mlt_u.ensure(sizeof(float) * (size_t)m.chains * kMltDims));
   PR_CUDA(c, c->mlt_cur.ensure(sizeof(float4) * (size_t)m.chains));
   PR_CUDA(c, c->mlt_acc.ensure(sizeof(float) * n3));
-  PR_CUDA(c, c->mlt_slots.ensure(mlt_scratch_bytes(m)));
+  PR_CUDA(c, ensure_scratch(c, g, c->mlt_slots, [&](const RenderCfg& q) { return mlt_scratch_bytes(q, m); }));
   PR_CUDA(c, cudaMemsetAsync(c->mlt_acc.p, 0, sizeof(float) * n3, c->stream));
   const DevScene& S = c->cur.dev;
   uint32_t* err = (uint32_t*)c->errword.p;
@@ -771,7 +788,7 @@ static int render_wavefront(pr_ctx* c, const RenderCfg& g, float* rgb_dev, int a
   // hold that, a smaller pool and passes of 4 M.
   uint64_t layers = 0, pass_cap = 0, frame_cap = 0;
   unsigned int P = 0, spawn_cap = 0;
-  for (bool less = false;; less = true) {
+  for (bool less = g.less != 0 || c->less_memory;; less = true) {
     const uint64_t max_pass = !sss ? (64ull << 20) : less ? (4ull << 20) : (16ull << 20);
     layers = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)g.spp, max_pass / wh));
     pass_cap = layers * wh;
@@ -796,6 +813,7 @@ static int render_wavefront(pr_ctx* c, const RenderCfg& g, float* rgb_dev, int a
       if (q.first && e == cudaSuccess) e = q.first->ensure(q.second);
     if (e == cudaErrorMemoryAllocation && !less) {
       cudaGetLastError();
+      c->less_memory = true;
       for (const auto& q : pool)
         if (q.first) q.first->release();
       continue;
@@ -889,6 +907,14 @@ static uint64_t frame_launches(const SceneObjData& sc, const RenderCfg& g) {
   return sc.worm.enabled || block_form(sc) ? 2 * pass_count(g) : 2;
 }
 
+// scratch of a frame outside of the wavefront form
+static size_t job_scratch_bytes(const SceneObjData& sc, const RenderCfg& g) {
+  if (sc.kerr.enabled) return kerr_scratch_bytes(sc.kerr, g);
+  if (sc.worm.enabled) return worm_scratch_bytes(g);
+  if (block_form(sc)) return plain_scratch_bytes(g);
+  return sizeof(float) * (size_t)g.width * g.height * 3 * (size_t)g.chunks;
+}
+
 int pr_render_dev(pr_ctx* c, const pr_camera* cam, const pr_render_params* p, float* rgb_dev, uint64_t sample_offset,
                   int accumulate) {
   if (!c) return PR_E_ARG;
@@ -910,11 +936,11 @@ int pr_render_dev(pr_ctx* c, const pr_camera* cam, const pr_render_params* p, fl
   if (kerr || worm) {
     // every scene query of a Kerr or wormhole scene is a geodesic trace: one form only
     if (kerr) {
-      PR_CUDA(c, c->partial.ensure(kerr_scratch_bytes(c->cur.kerr, g)));
+      PR_CUDA(c, ensure_scratch(c, g, c->partial, [&](const RenderCfg& q) { return kerr_scratch_bytes(c->cur.kerr, q); }));
       PR_CUDA(c, launch_kerr_render(c->cur.dev, c->cur.kerr, g, c->partial.p, rgb_dev, accumulate,
                                     (uint32_t*)c->errword.p, (unsigned long long*)c->counters.p, c->stream));
     } else {
-      PR_CUDA(c, c->partial.ensure(worm_scratch_bytes(g)));
+      PR_CUDA(c, ensure_scratch(c, g, c->partial, worm_scratch_bytes));
       PR_CUDA(c, launch_worm_render(c->cur.dev, c->cur.worm, g, c->partial.p, rgb_dev, accumulate,
                                     (uint32_t*)c->errword.p, (unsigned long long*)c->counters.p, c->stream));
     }
@@ -925,7 +951,7 @@ int pr_render_dev(pr_ctx* c, const pr_camera* cam, const pr_render_params* p, fl
     st = render_wavefront(c, g, rgb_dev, accumulate);
     if (st != PR_OK) return st;
   } else if (!c->cur.dev.has_sss) {
-    PR_CUDA(c, c->partial.ensure(plain_scratch_bytes(g)));
+    PR_CUDA(c, ensure_scratch(c, g, c->partial, plain_scratch_bytes));
     PR_CUDA(c, launch_plain(c->cur.dev, g, c->partial.p, rgb_dev, accumulate, (uint32_t*)c->errword.p,
                              (unsigned long long*)c->counters.p, c->stream));
   } else {
@@ -1012,7 +1038,7 @@ int pr_render_adjoint_dev(pr_ctx* c, const pr_camera* cam, const pr_render_param
   double* de = d_emission ? d_emission : (double*)c->adj_scratch.p + 3 * std::max(n_mat, 1);
   if (!d_color) PR_CUDA(c, cudaMemsetAsync(dc, 0, 3 * sizeof(double) * n_mat, c->stream));
   if (!d_emission) PR_CUDA(c, cudaMemsetAsync(de, 0, 3 * sizeof(double) * n_mat, c->stream));
-  PR_CUDA(c, c->adj_samples.ensure(adjoint_scratch_bytes(g, n_mat)));
+  PR_CUDA(c, ensure_scratch(c, g, c->adj_samples, [&](const RenderCfg& q) { return adjoint_scratch_bytes(q, n_mat); }));
   PR_CUDA(c, cudaMemsetAsync(c->errword.p, 0, 4, c->stream));
   PR_CUDA(c, cudaMemsetAsync(c->counters.p, 0, 128, c->stream));
   PR_CUDA(c, cudaEventRecord(c->ev0, c->stream));
@@ -1420,9 +1446,6 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
   PR_CUDA(c, cudaSetDevice(c->device));
   cudaGetLastError();  // an error left by an unrelated earlier call is not this call's
   std::vector<RenderCfg> cfg((size_t)n);
-  // the jobs of a branch run one after another and share its scratch
-  const int n_streams = std::min(n, 16);
-  std::vector<size_t> branch_room((size_t)n_streams, 0), off((size_t)n_streams + 1, 0);
   uint64_t paths = 0;
   bool all_kerr = true;
   for (int j = 0; j < n; j++) {
@@ -1437,14 +1460,6 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
     // the batch fills the GPU with many jobs: fewer sample chunks per job (subsurface scenes)
     cfg[j].chunks = std::max(1, std::min(cfg[j].chunks, (int)std::ceil(2.0e5 / ((double)cfg[j].width * cfg[j].height))));
     cfg[j].chunks = std::min(cfg[j].chunks, cfg[j].spp);
-    const SceneObjData& sc = J.scene->data;
-    size_t bytes = sizeof(float) * (size_t)cfg[j].width * cfg[j].height * 3 * (size_t)cfg[j].chunks;
-    if (J.params.mode == PR_MODE_WAVEFRONT && !sc.kerr.enabled && !sc.worm.enabled) bytes = 0;
-    else if (sc.kerr.enabled) bytes = kerr_scratch_bytes(sc.kerr, cfg[j]);
-    else if (sc.worm.enabled) bytes = worm_scratch_bytes(cfg[j]);
-    else if (block_form(sc)) bytes = plain_scratch_bytes(cfg[j]);
-    size_t& room = branch_room[j % n_streams];
-    room = std::max(room, (bytes + 255) / 256 * 256);
     paths += (uint64_t)cfg[j].spp * cfg[j].width * cfg[j].height;
   }
   // jobs in the wavefront form share the context's path pool: they run one
@@ -1453,8 +1468,20 @@ int pr_render_batch(pr_ctx* c, int n, const pr_job* jobs) {
   for (int j = 0; j < n; j++)
     wf_job[j] = jobs[j].params.mode == PR_MODE_WAVEFRONT && !jobs[j].scene->data.kerr.enabled &&
                 !jobs[j].scene->data.worm.enabled;
-  for (int k = 0; k < n_streams; k++) off[k + 1] = off[k] + branch_room[k];
-  PR_CUDA(c, c->batch_partial.ensure(std::max<size_t>(off[n_streams], 1)));
+  // the jobs of a branch run one after another and share its scratch
+  const int n_streams = std::min(n, 16);
+  std::vector<size_t> off((size_t)n_streams + 1, 0);
+  RenderCfg batch{};
+  batch.less = c->less_memory ? 1 : 0;
+  PR_CUDA(c, ensure_scratch(c, batch, c->batch_partial, [&](const RenderCfg& g) {
+    std::vector<size_t> room((size_t)n_streams, 0);
+    for (int j = 0; j < n; j++) {
+      cfg[j].less = g.less;
+      if (!wf_job[j]) room[j % n_streams] = std::max(room[j % n_streams], job_scratch_bytes(jobs[j].scene->data, cfg[j]));
+    }
+    for (int k = 0; k < n_streams; k++) off[k + 1] = off[k] + (room[k] + 255) / 256 * 256;
+    return std::max<size_t>(off[n_streams], 1);
+  }));
   while ((int)c->batch_streams.size() < n_streams) {
     cudaStream_t st;
     PR_CUDA(c, cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));

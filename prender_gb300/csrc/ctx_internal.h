@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+#include <cstdlib>
 #include <string>
 #include <vector>
 
@@ -16,17 +18,26 @@ namespace pr {
 struct DevBuf {
   void* p = nullptr;
   size_t n = 0;
+  inline static std::atomic<size_t> held{0};  // by all buffers of the process
   cudaError_t ensure(size_t bytes) {
     if (bytes <= n && p) return cudaSuccess;
-    if (p) cudaFree(p);
-    p = nullptr;
-    n = 0;
-    cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
-    if (e == cudaSuccess) n = bytes;
-    return e;
+    release();
+    // PR_DEVICE_MEMORY_MB: a bound on what the library holds (the rest of the
+    // device is another's); beyond it an allocation fails as on a full device
+    const char* e = getenv("PR_DEVICE_MEMORY_MB");
+    if (e && held + bytes > (size_t)strtoull(e, nullptr, 10) << 20) return cudaErrorMemoryAllocation;
+    const cudaError_t r = cudaMalloc(&p, bytes ? bytes : 16);
+    if (r != cudaSuccess) {
+      p = nullptr;
+      return r;
+    }
+    n = bytes;
+    held += n;
+    return r;
   }
   void release() {
     if (p) cudaFree(p);
+    held -= n;
     p = nullptr;
     n = 0;
   }
@@ -86,6 +97,7 @@ struct pr_ctx {
   unsigned int wf_graph_next = 0;    // the entry that the next new graph takes
   unsigned int tuned_slots = 0;      // autotuner's wavefront pool size (0: default)
   unsigned int tuned_trace_bps = 0;  // autotuner's traversal blocks per SM (0: default)
+  bool less_memory = false;          // an allocation of the usual size failed since the last upload
   bool force_host_loop = false;      // the autotuner times candidates with the host-driven loop
   // pr_render_batch
   cudaGraphExec_t batch_exec = nullptr;

@@ -1227,7 +1227,8 @@ __global__ void __launch_bounds__(128) kerr_render_kernel(const __grid_constant_
 // scratch of a frame: the samples of a pass, then the far records
 inline unsigned long long kerr_far_cap(const RenderCfg& cfg) {
   const unsigned long long n = pass_pixels(cfg) * (unsigned long long)cfg.spp;
-  return n < (1ull << 19) ? n : 1ull << 19;  // beyond that the near kernel goes on itself
+  const unsigned long long most = cfg.less ? 1ull << 15 : 1ull << 19;  // beyond that the near kernel goes on itself
+  return n < most ? n : most;
 }
 inline size_t kerr_bytes(const RenderCfg& cfg, bool far) {
   return pass_bytes(cfg) + (far ? sizeof(KerrFar) * (size_t)kerr_far_cap(cfg) : 0);

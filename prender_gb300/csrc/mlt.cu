@@ -345,7 +345,7 @@ BlockShape mlt_shape(unsigned long long n, int sms) {
 template <bool SEEDS>
 cudaError_t run_paths(const DevScene& S, const RenderCfg& cfg, MltRun R, unsigned long long n, void* scratch,
                       uint32_t* err, unsigned long long* counters, cudaStream_t stream) {
-  const BlockShape b = mlt_shape(n, sm_count());
+  const BlockShape b = mlt_shape(n, slot_sms(cfg));
   const size_t slots = (size_t)b.blocks * b.slots;
   char* p = static_cast<char*>(scratch);
   cudaError_t e = cudaMemsetAsync(p, 0, 256, stream);
@@ -364,10 +364,10 @@ cudaError_t run_paths(const DevScene& S, const RenderCfg& cfg, MltRun R, unsigne
 
 }  // namespace
 
-size_t mlt_scratch_bytes(const MltCfg& m) {
+size_t mlt_scratch_bytes(const RenderCfg& cfg, const MltCfg& m) {
   size_t most = 0;
   for (unsigned long long n : {(unsigned long long)m.seeds, (unsigned long long)m.chains}) {
-    const BlockShape b = mlt_shape(n, sm_count());
+    const BlockShape b = mlt_shape(n, slot_sms(cfg));
     const size_t slots = (size_t)b.blocks * b.slots;
     most = std::max(most, 512 + block_pool_bytes(slots) + 256 + 16 * slots);
   }

@@ -24,7 +24,7 @@ struct MltCfg {
 };
 
 // scratch of the launches below
-size_t mlt_scratch_bytes(const MltCfg& m);
+size_t mlt_scratch_bytes(const RenderCfg& cfg, const MltCfg& m);
 // bootstrap: seeds paths from fresh primary samples -> luminance, colour
 // and pixel of each
 cudaError_t launch_mlt_seeds(const DevScene& S, const RenderCfg& cfg, const MltCfg& m, float* lum, float4* path,

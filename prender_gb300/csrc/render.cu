@@ -342,7 +342,7 @@ cudaError_t launch_sum(const RenderCfg& cfg, const SamplePass& A, float* dst, in
 
 // blocks of the frame's largest pass, for all of its passes
 static BlockShape plain_shape(const RenderCfg& cfg) {
-  return block_shape(pass_pixels(cfg) * (unsigned long long)cfg.spp, sm_count());
+  return block_shape(pass_pixels(cfg) * (unsigned long long)cfg.spp, slot_sms(cfg));
 }
 
 size_t plain_scratch_bytes(const RenderCfg& cfg) {

@@ -26,6 +26,7 @@ struct RenderCfg {
   uint32_t tiles_x, tiles_y;
   uint64_t seed;
   uint64_t sample_offset;
+  int less;         // little device memory is left: smaller passes and pools
 };
 
 // A frame whose samples finish in any order (plain form, Kerr and wormhole
@@ -45,7 +46,8 @@ constexpr unsigned long long kPassSamples = 1ull << 24;
 inline unsigned long long pass_pixels(const RenderCfg& cfg) {
   const char* e = getenv("PR_PASS_SAMPLES");
   const long long v = e ? strtoll(e, nullptr, 10) : 0;
-  const unsigned long long most = v >= 1 && v < (long long)kPassSamples ? (unsigned long long)v : kPassSamples;
+  const unsigned long long full = cfg.less ? kPassSamples / 16 : kPassSamples;
+  const unsigned long long most = v >= 1 && v < (long long)full ? (unsigned long long)v : full;
   const unsigned long long px = (unsigned long long)cfg.width * cfg.height, n = most / (unsigned long long)cfg.spp;
   return n < 1 ? 1 : n < px ? n : px;
 }
@@ -85,6 +87,8 @@ inline int sm_count() {
     sms = 152;
   return sms;
 }
+// the SMs that blocks with path slots in device memory are spread over
+inline int slot_sms(const RenderCfg& cfg) { return cfg.less ? (sm_count() + 3) / 4 : sm_count(); }
 
 cudaError_t launch_megakernel(const DevScene& S, const RenderCfg& cfg, float* out, uint32_t* err,
                               unsigned long long* counters, cudaStream_t stream);
