@@ -1097,7 +1097,7 @@ struct KerrPathJob {
     }
     int x, y;
     uint32_t k;
-    pass_sample(cfg, F.pass, g, x, y, k);
+    pass_sample(cfg, F.pass, (uint32_t)g, x, y, k);
     float3 o, d;
     id = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
     item = (uint32_t)g;

@@ -221,12 +221,12 @@ struct PlainPaths {
       return false;
     }
     // a pixel's samples one after another: the first segments of a warp are close together
+    F.item[i] = (uint32_t)g;
     int x, y;
     uint32_t k;
-    pass_sample(cfg, F.pass, g, x, y, k);
+    pass_sample(cfg, F.pass, (uint32_t)g, x, y, k);
     float3 o, d;
     P.id[i] = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
-    F.item[i] = (uint32_t)g;
     root_path(ps, o, d);
     return true;
   }
@@ -246,6 +246,7 @@ struct PlainPaths {
                                         ShadowReq* sh, int& nsh) {
     PathState child;
     const unsigned long long id = P.id[i];
+    const uint32_t item = F.item[i];  // with the path's state: read where the path ends, its wait would show
     const int r = shade<false, FULL, FULL>(S, cfg, ps, hit, h, id, sh, nsh, child, err);
     // pending: waiting branches; bit 8: the sample has split
     if (r == SHADE_SPLIT) {
@@ -272,7 +273,7 @@ struct PlainPaths {
         return SHADE_CONTINUE;
       }
     }
-    F.pass.sample[F.item[i]] = finish_sample(cfg, L, err);
+    F.pass.sample[item] = finish_sample(cfg, L, err);
     paths++;
     return SHADE_END;
   }

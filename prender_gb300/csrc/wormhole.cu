@@ -478,7 +478,7 @@ struct WormPathJob {
     }
     int x, y;
     uint32_t k;
-    pass_sample(cfg, F, g, x, y, k);
+    pass_sample(cfg, F, (uint32_t)g, x, y, k);
     float3 o, d;
     id = camera_ray(cfg, x, y, cfg.sample_offset + (uint64_t)k, o, d);
     item = (uint32_t)g;
