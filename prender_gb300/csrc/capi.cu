@@ -649,25 +649,11 @@ static cudaError_t ensure_scratch(pr_ctx* c, RenderCfg& g, DevBuf& b, Bytes byte
 
 extern "C" {
 
-// Slots of the wavefront pool (paths in flight) for a pass of n camera
-// samples; PR_WF_SLOTS overrides, a tuned size bounds it.  Every iteration's
-// launches end with their longest rays on an emptying chip, so a large frame
-// takes a large pool: mesh Cornell box 1024x768 x 64 spp, 2^21 / 2^22 / 2^23
-// slots on GB300: 281 / 269 / 268 ms.  A pass should refill it about once
-// (n / 2: paths that start together also thin out together; 3.1 M glass
-// samples 45.1 / 42.2 / 43.9 ms at 2^19 / 2^20 / 2^22), or in subsurface
-// scenes, whose paths are longer, a few times (n / 4: 4 M of their samples
-// 38 / 37 / 40 ms at 2^19 / 2^20 / 2^21), but below 2^19 slots the
-// launches are too small to pay for themselves: 0.48 M samples 6.8 / 5.7 /
-// 5.5 ms at 2^17 / 2^18 / all at once.
-constexpr unsigned int kWfMinSlots = 1u << 19, kWfMaxSlots = 1u << 22, kWfSpareSlots = 1u << 21;
 static unsigned int wavefront_slots(uint64_t n, unsigned int tuned, bool sss) {
   const char* e = getenv("PR_WF_SLOTS");
   const long v = e ? strtol(e, nullptr, 10) : 0;
   if (v >= 1024 && v <= (1L << 24)) return tuned ? tuned : (unsigned int)v;
-  const uint64_t want = n <= kWfMinSlots ? (n + 8191) / 8192 * 8192 : (n / (sss ? 4 : 2) + 65535) / 65536 * 65536;
-  const uint64_t most = tuned ? tuned : sss ? kWfSpareSlots : kWfMaxSlots;
-  return (unsigned int)std::min(most, n <= kWfMinSlots ? want : std::max<uint64_t>(want, kWfMinSlots));
+  return wavefront_pool(n, tuned, sss);
 }
 
 // PR_MODE_MLT (Render::RunMLT's estimator as parallel chains, mlt.cu): the

@@ -78,6 +78,30 @@ struct WfLaunch {
   }
 };
 
+// Slots of the wavefront pool (paths in flight) for a pass of n camera
+// samples.  Every iteration's launches end with their longest rays on an
+// emptying chip, so a large frame takes a large pool: mesh Cornell box 1024x768 x 64 spp, 2^21 / 2^22 / 2^23
+// slots on GB300: 281 / 269 / 268 ms.  A pass should refill it about once
+// (n / 2: paths that start together also thin out together; 3.1 M glass
+// samples 45.1 / 42.2 / 43.9 ms at 2^19 / 2^20 / 2^22), or in subsurface
+// scenes, whose paths are longer, a few times (n / 4: 4 M of their samples
+// 38 / 37 / 40 ms at 2^19 / 2^20 / 2^21), but below 2^19 slots the
+// launches are too small to pay for themselves: 0.48 M samples 6.8 / 5.7 /
+// 5.5 ms at 2^17 / 2^18 / all at once.
+// A tuned size takes the place of these shares, as far as the pass has samples
+// for it (the tuner's own frames have samples for each of its candidates).
+constexpr unsigned int kWfMinSlots = 1u << 19, kWfMaxSlots = 1u << 22, kWfSpareSlots = 1u << 21;
+inline unsigned int wavefront_pool(uint64_t n, unsigned int tuned, bool sss) {
+  if (n <= kWfMinSlots) {
+    const uint64_t all = (n + 8191) / 8192 * 8192, most = tuned ? tuned : kWfMinSlots;
+    return (unsigned int)(all < most ? all : most);
+  }
+  const uint64_t share = tuned ? n : sss ? n / 4 : n / 2, most = tuned ? tuned : sss ? kWfSpareSlots : kWfMaxSlots;
+  uint64_t want = (share + 65535) / 65536 * 65536;
+  if (want < kWfMinSlots) want = kWfMinSlots;
+  return (unsigned int)(want < most ? want : most);
+}
+
 cudaError_t wf_set_constants(const DevScene& S, const RenderCfg& cfg, const WfBufs& B, cudaStream_t s);
 cudaError_t wf_reset_launch(unsigned int n_slots, cudaStream_t s);
 cudaError_t wf_build_graph(const WfLaunch& L, cudaStream_t s, cudaGraphExec_t* exec);

@@ -54,3 +54,8 @@ def test_segments_left_out_have_no_hit(tmp_path, length):
 def test_sphere_runs_are_the_fp64_tests_of_every_sphere(tmp_path, scene, length):
     r = _run(tmp_path, "sphere_runs", ["-O2"], [scene, length])
     assert r.returncode == 0, r.stdout + r.stderr[-3000:]
+
+
+def test_wavefront_pool_sizes(tmp_path):
+    r = _run(tmp_path, "wavefront_pool")
+    assert r.returncode == 0, r.stdout + r.stderr[-3000:]
