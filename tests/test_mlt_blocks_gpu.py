@@ -9,6 +9,7 @@ import pytest
 
 from prender_gb300 import _abi as A
 from prender_gb300 import gpu, scenes
+from prender_gb300.scene import Material, RenderSettings, Scene
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +41,33 @@ def test_chains_do_not_depend_on_their_slots(ctx, chains, mutations):
     # sums of at most k non-negative floats in any order
     k = 2 * chains * mutations
     np.testing.assert_allclose(a, b, rtol=2.0 * k * 2.0 ** -24, atol=0.0)
+
+
+@pytest.mark.parametrize("chains,mutations", [(1, 129), (913, 3), (19455, 2), (19456, 2), (65536, 1), (4096, 65),
+                                              (233473, 1)])
+def test_every_splat_counts_once(ctx, chains, mutations):
+    """Every path sees a background of radiance 1, so every proposal is taken
+    and splats once, with one weight or (a large step) twice that: a pixel is
+    a whole number of them, the same in every run, and their sum is that of
+    all proposals.  A pixel's n float splats are off by at most n^2 2^-24 of
+    one (n up to some 1500 here: 0.14); a lost or doubled one is off by 1."""
+    w, h = 32, 24
+    s = Scene()
+    s.camera = scenes.cornell_spheres(w, h, 1, 1).camera
+    s.background = (1.0, 1.0, 1.0)
+    p, d = np.array(s.camera.position), np.array(s.camera.dir)
+    s.add_sphere(tuple(p - 50.0 * d), 0.5, Material.diffuse((0.5, 0.5, 0.5)))  # behind the camera
+    st = s.settings = RenderSettings(samples=1, supersamples=1, mode=A.PR_MODE_MLT, seed=chains, pre_sample=3.0,
+                                     mutation=(chains * mutations + 0.5) / (w * h), mlt_chains=chains)
+    assert st.nee == 0
+    ctx.upload(s)
+    n = chains * mutations
+    counts = []
+    for _ in range(2):
+        img = ctx.render(s).astype(np.float64)
+        k = img * 1.5 * n / (w * h)  # a splat: (1 + large) / (1 / b + 1/2), b = 1
+        assert np.abs(k - np.rint(k)).max() < 0.25
+        counts += [np.rint(k[..., c]) for c in range(3)]  # each channel has its own order of additions
+    assert all(np.array_equal(k, counts[0]) for k in counts)
+    large = counts[0].sum() - n  # of n proposals, each with probability 1/2
+    assert abs(large - n / 2) <= 6.0 * np.sqrt(n / 4) + 1
