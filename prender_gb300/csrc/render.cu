@@ -294,38 +294,48 @@ __global__ void __launch_bounds__(kBlockThreads, 1)
 
 // Adds up the samples of n pixels from px0 on, g threads a pixel (a power of
 // two up to 32, or the whole block), times the sensor response
-// (render.h:1405-1409); accumulate != 0 adds to what dst holds.  12 bytes a
-// sample: 64 spp of 1024x768 in 0.2 ms of the frame's 360.
+// (render.h:1405-1409); accumulate != 0 adds to what dst holds.  Each sum is
+// two floats (two_add keeps every addition's error): right to some spp 2^-48
+// for a few FP32 instructions, where FP64 additions were bound by that pipe
+// (1.25 M samples of the mesh Cornell box 321x243: 55 -> 16 us).
 constexpr int kSumThreads = 256;
+struct Sum3 {
+  float s[3], e[3];
+};
+__device__ __forceinline__ void sum_add(Sum3& a, int c, float s, float e) {
+  two_add(a.s[c], a.e[c], s);
+  a.e[c] += e;
+}
 __global__ void __launch_bounds__(kSumThreads)
     sum_samples(const float3* __restrict__ sample, float* __restrict__ dst, int width, int height, uint32_t spp,
                 unsigned long long px0, unsigned long long n, uint32_t g, int accumulate, float sensor) {
-  __shared__ double part[kSumThreads / 32][3];
+  __shared__ Sum3 part[kSumThreads / 32];
   const unsigned long long t = (unsigned long long)blockIdx.x * kSumThreads + threadIdx.x, p = t / g;
   const uint32_t l = (uint32_t)(t - p * g);
-  double a[3] = {0.0, 0.0, 0.0};
+  Sum3 a = {};
   if (p < n)
     for (uint32_t k = l; k < spp; k += g) {
       const float3 v = sample[p * spp + k];
-      a[0] += (double)v.x;
-      a[1] += (double)v.y;
-      a[2] += (double)v.z;
+      sum_add(a, 0, v.x, 0.0f);
+      sum_add(a, 1, v.y, 0.0f);
+      sum_add(a, 2, v.z, 0.0f);
     }
   for (int off = (int)(g < 32 ? g : 32) / 2; off > 0; off >>= 1)
 #pragma unroll
-    for (int c = 0; c < 3; c++) a[c] += __shfl_down_sync(0xffffffffu, a[c], off);
+    for (int c = 0; c < 3; c++)
+      sum_add(a, c, __shfl_down_sync(0xffffffffu, a.s[c], off), __shfl_down_sync(0xffffffffu, a.e[c], off));
   if (g > 32) {
-    if ((threadIdx.x & 31) == 0)
-      for (int c = 0; c < 3; c++) part[threadIdx.x / 32][c] = a[c];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x / 32] = a;
     __syncthreads();
     for (int w = 1; w < kSumThreads / 32; w++)
-      for (int c = 0; c < 3; c++) a[c] += part[w][c];
+      for (int c = 0; c < 3; c++) sum_add(a, c, part[w].s[c], part[w].e[c]);
   }
   if (p >= n || l != 0) return;
   const unsigned long long px = px0 + p, y = px / (unsigned int)width, x = px - y * (unsigned int)width;
   float* o = dst + 3 * ((size_t)(height - 1 - (int)y) * width + (size_t)x);
   for (int c = 0; c < 3; c++) {
-    const float v = (float)a[c] * sensor;
+    // past the largest float the sum is infinite and its error no number
+    const float v = (isfinite(a.s[c]) ? a.s[c] + a.e[c] : a.s[c]) * sensor;
     o[c] = accumulate ? o[c] + v : v;
   }
 }

@@ -31,7 +31,7 @@ struct RenderCfg {
 
 // A frame whose samples finish in any order (plain form, Kerr and wormhole
 // frames): each leaves its radiance in its own place, pixel by pixel, and
-// sum_samples adds up a pixel's samples in FP64 in a fixed order, so the image
+// sum_samples adds up a pixel's samples in a fixed order, so the image
 // does not depend on the schedule and holds any finite value (sums in fixed
 // point wrap or lose what lies outside of their range).  A frame of more
 // samples than kPassSamples takes passes of whole pixels.
@@ -41,8 +41,8 @@ struct SamplePass {
   unsigned long long samples;  // of the pass
   unsigned long long px0;      // its first pixel (scan line order)
 };
-// 192 MB of samples (64 spp of 1024x768 in 3 passes 368.3 ms, in one of 604 MB
-// 366.9; fixed-point sums 363.6); PR_PASS_SAMPLES may lower it
+// 192 MB of samples; PR_PASS_SAMPLES may lower it.  A pass ends on an emptying
+// chip: 64 spp of 1024x768 in 3 passes 368.8 ms, some 0.8 less per pass saved
 constexpr unsigned long long kPassSamples = 1ull << 24;
 inline unsigned long long pass_pixels(const RenderCfg& cfg) {
   const char* e = getenv("PR_PASS_SAMPLES");

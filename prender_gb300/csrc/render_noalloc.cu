@@ -31,8 +31,8 @@
 // Sample chunks: each pixel's samples are split into min(ceil(1.2e6 / pixels),
 // spp) chunks, each summed by its own thread, or into as many as fit in the
 // array (for example one instead of two at 1024 x 768).  The samples are
-// pr_render_dev's, which adds them in FP64: images agree to float
-// rounding, not bit for bit.
+// pr_render_dev's, which adds them as pairs of floats: images agree to
+// float rounding, not bit for bit.
 #include <cuda_runtime.h>
 
 #include <mutex>
