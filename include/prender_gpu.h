@@ -457,10 +457,14 @@ int pr_trace_fast(pr_ctx* ctx, const double* rays, int64_t n, int32_t* entity, i
  * already multiplied by 1/(total samples) and by sensor_response.  With
  * sample_offset = 0 and accumulate = 0 the buffer is overwritten.
  * The plain form, Kerr and wormhole frames add samples as pairs of floats
- * (any finite radiance, right to some 2^-40 of the sum).  The
- * wavefront form adds them in fixed point of 2^-40 (a split or subsurface
- * sample's branches in 2^-32 before): its pixel sums have to stay below
- * 2^23, and what is not well above that step is lost. */
+ * (any finite radiance, right to some spp 2^-48 of the sum; plain subsurface
+ * scenes in float chunks).  The wavefront form adds them in fixed point of
+ * 2^-40 (a split or subsurface sample's branches in 2^-32 before): its pixel
+ * sums have to stay below 2^23, and what is not well above the step is lost.
+ * The calls keep scratch in the context (a frame's samples, path slots); where
+ * the device cannot hold the usual sizes they run with smaller ones until the
+ * next scene upload.  PR_DEVICE_MEMORY_MB in the environment bounds what the
+ * library holds. */
 int pr_render(pr_ctx* ctx, const pr_camera* cam, const pr_render_params* prm,
               float* rgb_accum, uint64_t sample_offset, int accumulate);
 int pr_render_dev(pr_ctx* ctx, const pr_camera* cam, const pr_render_params* prm,
@@ -483,9 +487,9 @@ int pr_render_dev(pr_ctx* ctx, const pr_camera* cam, const pr_render_params* prm
  * on the GPU share the array and race.  The scene must already be uploaded
  * with pr_scene_upload (which allocates, at set-up).  It traces the paths of
  * pr_render_dev, one thread per pixel and sample chunk; the image agrees with
- * pr_render_dev's to float rounding (pr_render_dev adds samples without
- * rounding errors to speak of, this call in min(ceil(1.2e6 / pixels), spp) float chunks, or in fewer where
- * their partial images would not fit in the array). */
+ * pr_render_dev's to float rounding (pr_render_dev adds samples as pairs of
+ * floats, this call in min(ceil(1.2e6 / pixels), spp) float chunks, or in
+ * fewer where their partial images would not fit in the array). */
 int pr_render_dev_noalloc(pr_ctx* ctx, const pr_camera* cam, const pr_render_params* prm, float* rgb_accum_dev,
                           uint64_t sample_offset, int accumulate);
 

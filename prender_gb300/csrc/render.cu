@@ -186,7 +186,7 @@ __global__ void reduce_chunks(const float* __restrict__ partial, float* __restri
 // Resident blocks take camera samples one by one, pixel by pixel
 // (block_paths.cuh), and leave each finished sample in its place of the pass
 // (sum_samples adds them up).  Bound by instruction issue and divergence; mesh Cornell
-// box 321x243 x 16 spp on GB300 37.7 ms in pt_megakernel, 8.5 here, spheres
+// box 321x243 x 16 spp on GB300 37.7 ms in pt_megakernel, 8.4 here, spheres
 // 256x192 x 16 (FP64 sphere tests) 16.8 -> 6.9, Ward 404x248 x 4 22.2 -> 6.1.
 // FULL: glossy lobes, other lights, textures; the same shade() instantiations
 // as pt_megakernel's, since contraction (and with it a path's last bits)

@@ -4,8 +4,9 @@
 // with a small local stack of node groups: children visited near to far by
 // their octant slots, each child box culled against the current closest hit,
 // leaves tested as soon as their node is visited.
-// Spheres keep the reference's FP64 test (its 1e5-radius walls cancel
-// catastrophically in FP32); planes and triangles are FP32.
+// Spheres that FP32 bounds cannot rule out take the reference's FP64 test
+// (its 1e5-radius walls cancel catastrophically in FP32); planes and
+// triangles are FP32.
 #pragma once
 #include "device_common.cuh"
 
